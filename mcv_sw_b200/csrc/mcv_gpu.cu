@@ -124,6 +124,8 @@ struct mcv_handle {
   float4 *bnd32 = nullptr;
   double4 *met1d = nullptr;
   double *phibar = nullptr;
+  double *sgm = nullptr;   // strip form: sqrtG of one panel
+  float2 *met2 = nullptr;  // strip form: {1/sqrtG, sqrtG f} of panels 1-4 and of panel 5
   double *prec = nullptr;  // TMA form: per (member, panel, tile) linear references of a step's first stage
   std::vector<double> phibar_host;
   // shared
@@ -178,7 +180,7 @@ struct Layout {
   size_t total = 0;
   size_t f64_state[9]{}, f64_acc[3]{}, mix_state[6]{}, mix_inc[6]{}, mix_acc[3]{};
   size_t metric[5]{}, phis = 0, phis32 = 0, bnd = 0, bnd32 = 0, M = 0, N = 0, iref = 0, coef = 0, partial = 0,
-         met1d = 0, phibar = 0, active = 0, flags = 0, err = 0, stage = 0, prec = 0, area = 0;
+         met1d = 0, sgm = 0, met2 = 0, phibar = 0, active = 0, flags = 0, err = 0, stage = 0, prec = 0, area = 0;
 };
 
 Layout make_layout(const GridDesc &g, int H, int scheme, int precision, int members) {
@@ -205,6 +207,8 @@ Layout make_layout(const GridDesc &g, int H, int scheme, int precision, int memb
     L.phis32 = take(f32);
     L.bnd32 = take(sizeof(float4) * 24 * (size_t)g.n * members);
     L.met1d = take(sizeof(double4) * (size_t)g.np);
+    L.sgm = take(sizeof(double) * (size_t)g.plane);
+    L.met2 = take(sizeof(float2) * 2 * (size_t)g.plane);
     L.phibar = take(sizeof(double) * members);
     // 96-byte linear-reference records for the most tiles any candidate shape makes
     int ncand = 0, most = 0;
@@ -236,6 +240,31 @@ __global__ void repack_kernel(double *dst, const double *src, int cols, int dpit
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const long long r = blockIdx.y;
   if (c < cols) dst[r * dpitch + c] = src[r * spitch + c];
+}
+
+// The metric planes of the strip form from the 1-D table {tan, cos^2/R^2,
+// sin cos/R, R sec^2} (projection_mod.F90:150-211): sqrtG of one panel, and
+// {1/sqrtG, sqrtG f} of panels 1-4 (f = 2 Omega tan y / rho) and of panel 5
+// (f = 2 Omega / rho).
+__global__ void metric_planes_kernel(int np, int P, const double4 *met, double r2, double two_omega, double *sgm,
+                                     float2 *met2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  if (i >= np) return;
+  const double4 mx = met[i], my = met[j];
+  const double rho2 = 1. + mx.x * mx.x + my.x * my.x, rinv = 1. / sqrt(rho2);
+  const double sg = mx.w * my.w * (rinv * rinv * rinv);
+  const float rsg = (float)((rho2 * rho2 * rinv) * ((mx.y * my.y) * r2));
+  const long long o = (long long)j * P + i;
+  sgm[o] = sg;
+  met2[o] = make_float2(rsg, (float)(sg * (two_omega * (my.x * rinv))));
+  met2[(long long)np * P + o] = make_float2(rsg, (float)(sg * (two_omega * rinv)));
+}
+
+int build_metric_planes(mcv_handle *h) {
+  metric_planes_kernel<<<dim3((h->npx + 127) / 128, h->npx), 128, 0, h->stream>>>(
+      h->npx, h->g.P, h->met1d, h->radius * h->radius, 2. * kOmega, h->sgm, h->met2);
+  MCV_CUDA(cudaGetLastError(), "metric planes");
+  return MCV_OK;
 }
 
 // Copy a host array in the reference's padded Fortran layout (npx*npx*6,
@@ -316,6 +345,7 @@ StageArgs stage_args(mcv_handle *h, int s, int c) {
   a.uo = Yn[0]; a.vo = Yn[1]; a.po = Yn[2];
   a.fU = h->facc[0]; a.fV = h->facc[1]; a.fP = h->facc[2];
   a.phis32 = h->phis32; a.met1d = h->met1d; a.phibar = h->phibar; a.bnd32 = h->bnd32; a.prec = h->prec;
+  a.sgm = h->sgm; a.met2 = h->met2;
   a.two_omega = 2. * kOmega;
   a.r2 = h->radius * h->radius;
   float *const *din = nullptr, *const *dout = nullptr;
@@ -470,6 +500,30 @@ int stage_maps(mcv_handle *h, const StageLauncher &L, const StageArgs &a, int ki
   return MCV_OK;
 }
 
+// Tensor maps of a strip-form launch: boxes of a warp's row width and one cell row.
+int strip_maps(mcv_handle *h, const StageLauncher &L, const StageArgs &a, int kind, TileMaps &tm) {
+  const long long per_member = (long long)h->members * 6 * h->g.np;
+  const int bx = L.box_x, by = L.box_y;
+  int rc;
+  const double *f64[3] = {a.yu, a.yv, a.yp};
+  for (int k = 0; k < 3; ++k)
+    if ((rc = encode_field(&tm.f[k], f64[k], false, h->g, per_member, bx, by))) return rc;
+  if ((rc = encode_field(&tm.f[3], a.sgm, false, h->g, h->g.np, bx, by))) return rc;
+  if ((rc = encode_field(&tm.f[4], a.phis32, true, h->g, per_member, bx, by))) return rc;
+  if (!first_stage(kind)) {
+    const float *f32[3] = {a.du, a.dv, a.dp};
+    for (int k = 0; k < 3; ++k)
+      if ((rc = encode_field(&tm.f[5 + k], f32[k], true, h->g, per_member, bx, by))) return rc;
+  }
+  if ((rc = encode_field(&tm.f[8], a.met2, false, h->g, 2LL * h->g.np, bx, by))) return rc;
+  if (kind == RK4_S2 || kind == RK4_S3 || kind == RK4_S4) {
+    const float *acc[3] = {a.fU, a.fV, a.fP};
+    for (int k = 0; k < 3; ++k)
+      if ((rc = encode_field(&tm.f[9 + k], acc[k], true, h->g, per_member, bx, by))) return rc;
+  }
+  return MCV_OK;
+}
+
 // Grid k of a stage launch: the handle's grid descriptor with the candidate's
 // tiles, its stage arguments, tensor maps and work items (edge-free ones first).
 template <int NB>
@@ -484,7 +538,8 @@ int add_grid(StageBatch<NB> &b, int k, mcv_handle *h, const StageLauncher &L, in
   std::memset(&tm, 0, sizeof(tm));
   tm.total = g.tiles_x * g.tiles_y * 6 * h->n_active;  // work items (tile, panel, member)
   if (L.tma)
-    if (int rc = stage_maps(h, L, b.a[k], stage_kind(h, s), tm)) return rc;
+    if (int rc = L.strip[0] ? strip_maps(h, L, b.a[k], stage_kind(h, s), tm) : stage_maps(h, L, b.a[k], stage_kind(h, s), tm))
+      return rc;
   return MCV_OK;
 }
 
@@ -507,19 +562,65 @@ void number_items(StageBatch<NB> &b, int n) {
   b.total = nin + ned;
 }
 
+// Strips of a strip-form launch over b's first n grids on `warps` resident
+// warps: every grid's columns of at most kStripCells cells are cut into
+// segments of about the same number of cell rows, as many as give the least
+// (passes over the warps) x (rows of a segment + what a segment pays for its
+// two halo rows and its start).
+template <int NB>
+void cut_strips(StageBatch<NB> &b, int n, int warps) {
+  constexpr double kStart = 2.0;
+  int most = 1;
+  for (int k = 0; k < n; ++k) {
+    b.nsx[k] = (b.g[k].Nc + kStripCells - 1) / kStripCells;
+    most = std::max(most, b.g[k].Nc);
+  }
+  double best = 1e300;
+  int rows = 1;
+  for (int len = 1; len <= most; ++len) {
+    long long strips = 0;
+    for (int k = 0; k < n; ++k) strips += 6LL * b.slots[k] * b.nsx[k] * ((b.g[k].Nc + len - 1) / len);
+    const double cost = (double)((strips + warps - 1) / warps) * (len + kStart);
+    if (cost < best) {
+      best = cost;
+      rows = len;
+    }
+  }
+  b.ngrids = n;
+  b.total = 0;
+  for (int k = 0; k < n; ++k) {
+    b.sy[k] = (b.g[k].Nc + rows - 1) / rows;
+    b.s0[k] = b.total;
+    b.total += 6 * b.slots[k] * b.nsx[k] * b.sy[k];
+  }
+  b.s0[n] = b.total;
+}
+
+// Blocks of a persistent launch over b's first n grids, whose work it numbers.
+template <int NB>
+int plan_persistent(StageBatch<NB> &b, int n, const StageLauncher &L, int kind, int resident) {
+  const int wpb = L.strip[kind];
+  if (!wpb) {
+    number_items(b, n);
+    return std::max(1, std::min(b.total, resident));
+  }
+  cut_strips(b, n, resident * wpb);
+  return std::max(1, std::min(b.total, resident));
+}
+
 int launch_stage(mcv_handle *h, int cand, int s, int c, bool pdl = true) {
   const StageLauncher &L = h->cands[cand];
   StageBatch<1> b;
   std::memset(&b, 0, sizeof(b));
   if (int rc = add_grid(b, 0, h, L, s, c)) return rc;
-  number_items(b, 1);
   const int kind = stage_kind(h, s);
   const StageLaunchFn launch = h->active_ident ? L.launch_ident[kind] : L.launch[kind];
   if (!L.tma) {
+    number_items(b, 1);
     launch(dim3(b.g[0].tiles_x * b.g[0].tiles_y, 6, h->n_active), h->stream, b, pdl);
     return MCV_OK;
   }
-  const int ctas = std::max(1, std::min(b.total, h->bps[cand] * h->nsm));
+  const int ctas = plan_persistent(b, 1, L, kind, h->bps[cand] * h->nsm);
   launch(dim3(ctas), h->stream, b, pdl);
   return MCV_OK;
 }
@@ -751,6 +852,8 @@ extern "C" int mcv_create(int order, int nc, int scheme, int precision, double d
     h->phis32 = (float *)(base + L.phis32);
     h->bnd32 = (float4 *)(base + L.bnd32);
     h->met1d = (double4 *)(base + L.met1d);
+    h->sgm = (double *)(base + L.sgm);
+    h->met2 = (float2 *)(base + L.met2);
     h->phibar = (double *)(base + L.phibar);
     h->prec = (double *)(base + L.prec);
   }
@@ -891,6 +994,7 @@ extern "C" int mcv_set_geometry(mcv_handle *h, const double *sqrtG, const double
   if (h->mixed)
     MCV_CUDA(cudaMemcpyAsync(h->met1d, met.data(), sizeof(double4) * npx, cudaMemcpyHostToDevice, h->stream),
              "upload metric table");
+  if (h->mixed && (rc = build_metric_planes(h))) return rc;
   MCV_CUDA(cudaStreamSynchronize(h->stream), "geometry upload");
   h->sqrtG_host.assign(sqrtG, sqrtG + NP);
   h->geometry_set = true;
@@ -926,6 +1030,8 @@ extern "C" int mcv_set_geometry_equiangular(mcv_handle *h) {
   MCV_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "clear error flag");
   if (int e = build_geometry_device(a, h->stream))
     return fail(MCV_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
+  if (h->mixed)
+    if (int rc = build_metric_planes(h)) return rc;
   int bad = 0;
   MCV_CUDA(cudaMemcpyAsync(&bad, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "read error flag");
   MCV_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "clear error flag");
@@ -1627,8 +1733,7 @@ int enqueue_group_stage(mcv_group *g, const std::vector<mcv_handle *> &act, cons
   std::memset(&b, 0, sizeof(b));
   for (size_t k = 0; k < act.size(); ++k)
     if (int rc = add_grid(b, (int)k, act[k], L, s, curs[k])) return rc;
-  number_items(b, (int)act.size());
-  const int ctas = std::max(1, std::min(b.total, g->bps * act[0]->nsm));
+  const int ctas = plan_persistent(b, (int)act.size(), L, stage_kind(act[0], s), g->bps * act[0]->nsm);
   L.launch_batch[stage_kind(act[0], s)](dim3(ctas), g->stream, b, true);
   launch_halo_batch<kMaxGrids>(act.data(), curs.data(), (int)act.size(), s, g->stream);
   return MCV_OK;

@@ -77,6 +77,8 @@ struct StageArgs {
   const double *phibar;       // mean depth per member
   float4 *bnd32;              // raw boundary copy of the increment
   double *prec;  // TMA form: linear references of the step's first stage per (member, panel, tile), 12 words each
+  const double *sgm;    // strip form: sqrtG of one panel [np][P] (the same on all six)
+  const float2 *met2;   // strip form: {1/sqrtG, sqrtG f} of panels 1-4 [np][P], then of panel 5 (panel 6: -f)
   double two_omega;
   double r2;  // radius squared (split precision: 1/sqrtG from the 1-D tables)
   float wd, wt;  // increment = wd * (input increment) + wt * tendency (RK3/RK4 weights)
@@ -90,6 +92,8 @@ struct StageArgs {
 // that with programmatic dependent launch the edge-free items of every grid
 // start while the previous halo kernels still run.
 constexpr int kMaxGrids = 4;
+// strip form: owned cells per strip, lanes 1..29 (lane 31 lends its first point to lane 30)
+constexpr int kStripCells = 29;
 template <int NB>
 struct StageBatch {
   TileMaps tm[NB];  // tensor maps of each grid's staged fields (TMA form)
@@ -101,6 +105,9 @@ struct StageBatch {
   int in0[NB + 1];  // first edge-free item of each grid
   int ed0[NB + 1];  // first edge item of each grid, counted from nin
   int slots[NB];    // active members of each grid
+  // strip form: columns of at most kStripCells cells, segments of cell rows and
+  // the first strip of each grid
+  int nsx[NB], sy[NB], s0[NB + 1];
 };
 
 // ---------------------------------------------------------------------------
@@ -1566,6 +1573,7 @@ struct StageLauncher {
   StageBatchFn launch_batch[7];  // up to kMaxGrids grids in one launch (TMA form; else null)
   cudaError_t (*prepare)();      // raises the dynamic shared-memory limit of every kind
   int (*blocks_per_sm)();        // resident CTAs per SM (sizes the persistent grid)
+  int strip[7];                  // strip form (mcv_strip.cuh): warps per block of each kind; else 0
 };
 
 template <int D, int CX, int CY, int NT, int MINB, bool MIXED, int WALK, bool TMA = false, int OPT = 0>
@@ -1650,7 +1658,7 @@ struct StageConfig {
                     {&launch<0>, &launch<1>, &launch<2>, &launch<3>, &launch<4>, &launch<5>, &launch<6>},
                     {&launch_ident<0>, &launch_ident<1>, &launch_ident<2>, &launch_ident<3>, &launch_ident<4>,
                      &launch_ident<5>, &launch_ident<6>},
-                    {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}, &prepare, &blocks_per_sm};
+                    {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}, &prepare, &blocks_per_sm, {0, 0, 0, 0, 0, 0, 0}};
     if constexpr (TMA) {
       StageBatchFn fb[7] = {&launch_batch<0>, &launch_batch<1>, &launch_batch<2>, &launch_batch<3>,
                             &launch_batch<4>, &launch_batch<5>, &launch_batch<6>};

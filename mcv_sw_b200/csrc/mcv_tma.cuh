@@ -19,8 +19,10 @@ namespace mcv {
 // Input fields of one stage launch, in the order the kernel stages them.
 // FP64 policy: us, vs, ps, phis, sqrtG, ig11, ig12, ig22.
 // Split precision: yu, yv, yp (FP64), phis32, du, dv, dp (FP32).
+// Strip form: yu, yv, yp, sqrtG of one panel (FP64), phis32, du, dv, dp (FP32),
+// met2 (8-byte pairs), the RK4 sums fU, fV, fP (FP32).
 struct TileMaps {
-  CUtensorMap f[8];
+  CUtensorMap f[12];
   int total;  // work items of the launch: tiles x 6 panels x active members
   int pad[15];
 };

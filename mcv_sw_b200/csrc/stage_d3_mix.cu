@@ -9,6 +9,8 @@
 
 namespace mcv {
 
+StageLauncher strip_launcher_d3();  // stage_strip_mix.cu
+
 const StageLauncher *stage_launchers_d3_mix(int *count) {
   static const StageLauncher table[] = {
     StageConfig<3, 12, 12, 320, 2, true, 0>::make(),
@@ -18,7 +20,8 @@ const StageLauncher *stage_launchers_d3_mix(int *count) {
     StageConfig<3, 16, 12, 448, 2, true, 0>::make(),
     StageConfig<3, 12, 12, 320, 2, true, 0, true>::make(),
     StageConfig<3, 12, 12, 320, 2, true, 2, true, 2>::make(),
-    StageConfig<3, 12, 12, 320, 2, true, 3, true, 3>::make()};
+    StageConfig<3, 12, 12, 320, 2, true, 3, true, 3>::make(),
+    strip_launcher_d3()};
   *count = (int)(sizeof(table) / sizeof(table[0]));
   return table;
 }

@@ -9,6 +9,8 @@
 
 namespace mcv {
 
+StageLauncher strip_launcher_d4();  // stage_strip_mix.cu
+
 const StageLauncher *stage_launchers_d4_mix(int *count) {
   static const StageLauncher table[] = {
     StageConfig<4, 8, 8, 320, 2, true, 0>::make(),
@@ -17,7 +19,8 @@ const StageLauncher *stage_launchers_d4_mix(int *count) {
     StageConfig<4, 8, 8, 320, 2, true, 2>::make(),
     StageConfig<4, 8, 8, 256, 2, true, 0, true>::make(),
     StageConfig<4, 8, 8, 320, 2, true, 0, true>::make(),
-    StageConfig<4, 8, 8, 320, 2, true, 2, true, 3>::make()};
+    StageConfig<4, 8, 8, 320, 2, true, 2, true, 3>::make(),
+    strip_launcher_d4()};
   *count = (int)(sizeof(table) / sizeof(table[0]));
   return table;
 }

@@ -1,0 +1,10 @@
+// stage_strip_d4.cu -- the strip form of the stage kernel for MCV4, split
+// precision.  Compiled without FMA contraction: its fused operations are
+// written out, so that one grid and several grids in a launch give the same bits.
+#include "mcv_strip.cuh"
+
+namespace mcv {
+
+StageLauncher strip_launcher_d4() { return StripConfig<4>::make(); }
+
+}  // namespace mcv
