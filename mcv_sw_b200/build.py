@@ -11,13 +11,12 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 HOST_CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 SOURCES = ["mcv_gpu.cu", "stage_d3_f64.cu", "stage_d3_mix.cu", "stage_d4_f64.cu", "stage_d4_mix.cu",
-           "stage_strip_d3.cu", "stage_strip_d4.cu",
+           "stage_strip_d3_mix.cu", "stage_strip_d3_f64.cu", "stage_strip_d4_mix.cu", "stage_strip_d4_f64.cu",
            "mcv_geometry.cu", "mcv_diag.cu", "mcv_noalloc.cu", "host_setup.cpp", "mcv_server.cpp"]
 # per-source flags: the device geometry restates host formulas compiled
 # without FMA contraction; the strip kernels write their fused operations out
-SOURCE_FLAGS = {"mcv_geometry.cu": ["-fmad=false"], "stage_strip_d3.cu": ["-fmad=false"],
-                "stage_strip_d4.cu": ["-fmad=false"]}
-HEADERS = ["mcv_stage.cuh", "mcv_strip.cuh", "mcv_halo.cuh", "mcv_tma.cuh", "mcv_ksum.cuh", "mcv_internal.h", os.path.join("..", "..", "include", "mcv_gpu.h")]
+SOURCE_FLAGS = {src: ["-fmad=false"] for src in SOURCES if src == "mcv_geometry.cu" or src.startswith("stage_strip_")}
+HEADERS = ["mcv_stage.cuh", "mcv_strip.cuh", "mcv_strip64.cuh", "mcv_strip_table.cuh", "mcv_halo.cuh", "mcv_tma.cuh", "mcv_ksum.cuh", "mcv_internal.h", os.path.join("..", "..", "include", "mcv_gpu.h")]
 OBJ_DIR = os.path.join(HERE, "_lib", "obj")
 
 NVCC_FLAGS = [

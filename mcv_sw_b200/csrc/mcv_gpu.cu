@@ -130,6 +130,7 @@ struct mcv_handle {
   std::vector<double> phibar_host;
   // shared
   double *sqrtG = nullptr, *ig11 = nullptr, *ig12 = nullptr, *ig22 = nullptr, *fcor = nullptr, *phis = nullptr;
+  double *rsg = nullptr, *sgf = nullptr;  // FP64 strip form: 1/sqrtG and sqrtG f
   double4 *bnd = nullptr, *Mtab = nullptr, *Ntab = nullptr;
   int *giref = nullptr;
   double2 *gcoef = nullptr;
@@ -179,7 +180,7 @@ void grid_desc(int order, int nc, GridDesc &g, int &H, int &npx) {
 struct Layout {
   size_t total = 0;
   size_t f64_state[9]{}, f64_acc[3]{}, mix_state[6]{}, mix_inc[6]{}, mix_acc[3]{};
-  size_t metric[5]{}, phis = 0, phis32 = 0, bnd = 0, bnd32 = 0, M = 0, N = 0, iref = 0, coef = 0, partial = 0,
+  size_t metric[5]{}, rsg = 0, sgf = 0, phis = 0, phis32 = 0, bnd = 0, bnd32 = 0, M = 0, N = 0, iref = 0, coef = 0, partial = 0,
          met1d = 0, sgm = 0, met2 = 0, phibar = 0, active = 0, flags = 0, err = 0, stage = 0, prec = 0, area = 0;
 };
 
@@ -196,6 +197,8 @@ Layout make_layout(const GridDesc &g, int H, int scheme, int precision, int memb
   };
   const bool rk4 = scheme == MCV_RK4;
   if (precision == MCV_FP64) {
+    L.rsg = take(plane6);
+    L.sgf = take(plane6);
     for (int k = 0; k < 9; ++k) L.f64_state[k] = take(f64);
     if (rk4)
       for (int k = 0; k < 3; ++k) L.f64_acc[k] = take(f64);
@@ -260,7 +263,22 @@ __global__ void metric_planes_kernel(int np, int P, const double4 *met, double r
   met2[(long long)np * P + o] = make_float2(rsg, (float)(sg * (two_omega * rinv)));
 }
 
+// The FP64 strip form's planes: 1/sqrtG and sqrtG f of all six panels.
+__global__ void metric_planes64_kernel(int np, int P, const double *sqrtG, const double *f, double *rsg, double *sgf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= np) return;
+  const long long o = ((long long)blockIdx.z * np + blockIdx.y) * P + i;
+  rsg[o] = 1. / sqrtG[o];
+  sgf[o] = sqrtG[o] * f[o];
+}
+
 int build_metric_planes(mcv_handle *h) {
+  if (!h->mixed) {
+    metric_planes64_kernel<<<dim3((h->npx + 127) / 128, h->npx, 6), 128, 0, h->stream>>>(
+        h->npx, h->g.P, h->sqrtG, h->fcor, h->rsg, h->sgf);
+    MCV_CUDA(cudaGetLastError(), "metric planes");
+    return MCV_OK;
+  }
   metric_planes_kernel<<<dim3((h->npx + 127) / 128, h->npx), 128, 0, h->stream>>>(
       h->npx, h->g.P, h->met1d, h->radius * h->radius, 2. * kOmega, h->sgm, h->met2);
   MCV_CUDA(cudaGetLastError(), "metric planes");
@@ -314,6 +332,7 @@ int stage_kind(const mcv_handle *h, int s) { return (h->scheme == MCV_RK3_TVD ? 
 StageArgs stage_args(mcv_handle *h, int s, int c) {
   StageArgs a{};
   a.sqrtG = h->sqrtG; a.ig11 = h->ig11; a.ig12 = h->ig12; a.ig22 = h->ig22; a.fcor = h->fcor;
+  a.rsg = h->rsg; a.sgf = h->sgf;
   a.phis = h->phis;
   a.bnd = h->bnd;
   a.active = h->active;
@@ -505,6 +524,14 @@ int strip_maps(mcv_handle *h, const StageLauncher &L, const StageArgs &a, int ki
   const long long per_member = (long long)h->members * 6 * h->g.np;
   const int bx = L.box_x, by = L.box_y;
   int rc;
+  if (!h->mixed) {
+    if ((rc = stage_maps(h, L, a, kind, tm))) return rc;
+    const double *f[8] = {a.rsg, a.sgf, a.u0, a.v0, a.p0, a.aU, a.aV, a.aP};
+    const int nf = (kind == RK4_S2 || kind == RK4_S3 || kind == RK4_S4) ? 8 : 5;
+    for (int k = 0; k < nf; ++k)
+      if ((rc = encode_field(&tm.f[8 + k], f[k], false, h->g, k < 2 ? 6LL * h->g.np : per_member, bx, by))) return rc;
+    return MCV_OK;
+  }
   const double *f64[3] = {a.yu, a.yv, a.yp};
   for (int k = 0; k < 3; ++k)
     if ((rc = encode_field(&tm.f[k], f64[k], false, h->g, per_member, bx, by))) return rc;
@@ -857,6 +884,10 @@ extern "C" int mcv_create(int order, int nc, int scheme, int precision, double d
     h->phibar = (double *)(base + L.phibar);
     h->prec = (double *)(base + L.prec);
   }
+  if (!h->mixed) {
+    h->rsg = (double *)(base + L.rsg);
+    h->sgf = (double *)(base + L.sgf);
+  }
   h->sqrtG = (double *)(base + L.metric[0]);
   h->ig11 = (double *)(base + L.metric[1]);
   h->ig12 = (double *)(base + L.metric[2]);
@@ -994,7 +1025,7 @@ extern "C" int mcv_set_geometry(mcv_handle *h, const double *sqrtG, const double
   if (h->mixed)
     MCV_CUDA(cudaMemcpyAsync(h->met1d, met.data(), sizeof(double4) * npx, cudaMemcpyHostToDevice, h->stream),
              "upload metric table");
-  if (h->mixed && (rc = build_metric_planes(h))) return rc;
+  if ((rc = build_metric_planes(h))) return rc;
   MCV_CUDA(cudaStreamSynchronize(h->stream), "geometry upload");
   h->sqrtG_host.assign(sqrtG, sqrtG + NP);
   h->geometry_set = true;
@@ -1030,8 +1061,7 @@ extern "C" int mcv_set_geometry_equiangular(mcv_handle *h) {
   MCV_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "clear error flag");
   if (int e = build_geometry_device(a, h->stream))
     return fail(MCV_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
-  if (h->mixed)
-    if (int rc = build_metric_planes(h)) return rc;
+  if (int rc = build_metric_planes(h)) return rc;
   int bad = 0;
   MCV_CUDA(cudaMemcpyAsync(&bad, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "read error flag");
   MCV_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "clear error flag");

@@ -60,6 +60,7 @@ struct StageArgs {
   double *uo, *vo, *po;        // stage output (interior written here)
   double *aU, *aV, *aP;        // RK4 tendency accumulators
   const double *sqrtG, *ig11, *ig12, *ig22, *fcor;  // metric planes [6][np][P]
+  const double *rsg, *sgf;                          // strip form: 1/sqrtG and sqrtG f
   const double *phis;                               // [M][6][np][P]
   double4 *bnd;  // raw boundary copy [M][6][4][n] {u, v, phi, 0}
   double inc;    // dt or dt/2 (update_stat's inc_t) or the RK3 tendency weight

@@ -29,6 +29,41 @@
 namespace mcv {
 
 
+// one lane of the (converged) warp, which the compiler knows to be one
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n"
+      " .reg .pred p;\n"
+      " elect.sync _|p, 0xffffffff;\n"
+      " selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+// Strip s of a launch (grid k): cells [c0, c0 + w) of cell rows [r0, r1) of one
+// panel of one active member.  Panels vary fastest: split precision's six
+// panels share the metric planes.
+struct Strip {
+  int c0, w, r0, r1, panel, slot;
+};
+template <int NB>
+__device__ __forceinline__ Strip decode_strip(const StageBatch<NB> &b, int s, int k) {
+  const int Nc = b.g[k].Nc, nsx = b.nsx[k], sy = b.sy[k];
+  const int local = s - b.s0[k], per = 6 * b.slots[k];
+  const int q = local / per, pm = local - q * per;
+  Strip t;
+  t.slot = pm / 6;
+  t.panel = pm - 6 * t.slot;
+  const int seg = q / nsx, col = q - seg * nsx;
+  t.c0 = Nc * col / nsx;
+  t.w = Nc * (col + 1) / nsx - t.c0;
+  t.r0 = Nc * seg / sy;
+  t.r1 = Nc * (seg + 1) / sy;
+  return t;
+}
+
 // Shared memory of one warp for stage kind KIND: the staged input of a cell row
 // ([field][H rows][RE] each), the operands and results of the update of the
 // cell row before, the strip's metric entries in x, and the x sweep's results.
@@ -181,15 +216,9 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     const GridDesc &g = b.g[k];
     const StageArgs &a = b.a[k];
     const TileMaps &tm = b.tm[k];
-    // strip -> (segment of cell rows, column of cells, member, panel), panels fastest: the six
-    // panels share the metric planes
-    const int local = s - b.s0[k], per = 6 * b.slots[k];
-    const int q = local / per, pm = local - q * per;
-    const int slot = pm / 6, panel = pm - 6 * slot;
-    const int seg = q / b.nsx[k], col = q - seg * b.nsx[k];
-    const int c0 = g.Nc * col / b.nsx[k], w = g.Nc * (col + 1) / b.nsx[k] - c0;
-    const int r0 = g.Nc * seg / b.sy[k], r1 = g.Nc * (seg + 1) / b.sy[k];
-    const int mem = IDENT ? slot : active_member(a.active, a.ident, slot);
+    const Strip st = decode_strip(b, s, k);
+    const int c0 = st.c0, w = st.w, r0 = st.r0, r1 = st.r1, panel = st.panel;
+    const int mem = IDENT ? st.slot : active_member(a.active, a.ident, st.slot);
     const int X0 = c0 * H;  // padded index of lane 0's first point
     const int X0a = X0 & ~3, rem = X0 - X0a;
     const long long fbase = (long long)mem * g.mstride + (long long)panel * g.plane;
@@ -204,7 +233,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
       xt[lane * H + i] = m.x;
       xt[RP + lane * H + i] = m.y;
     }
-    const double phibar = a.phibar[mem], r2 = a.r2;
+    const double r2 = a.r2;
     if (!waited) {
       wait_prerequisite_grid();  // the halo kernel before
       waited = true;
@@ -300,8 +329,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         const double cv = rho2 * __fma_rn(sxy, u, my.y * v);
         o.u[i] = u;
         o.v[i] = v;
-        // E = phi + phi_s + K
-        o.e[i] = __fma_rn(0.5, __fma_rn(cv, v, cu * u), (p - phibar) + (double)psf[at + i]);
+        // E = phi + phi_s + K (differenced below, so no mean depth is taken off)
+        o.e[i] = __fma_rn(0.5, __fma_rn(cv, v, cu * u), p + (double)psf[at + i]);
         o.pg[i] = (float)(p * sgf[at + i]);
         o.cu[i] = (float)cu;
         o.cv[i] = (float)cv;
@@ -328,7 +357,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     float bE1[H], bE2[H], bM1[H], bM2[H], bU1[H], bU2[H];
 
     int sl = 0;  // the slot of the current cell row, where there are two
-    if (lane == 0) {
+    if (elect_one()) {
       fence_proxy_async();
       // the first row of the lower halo cell, then its block
       const int row = r0 * H, nel = min(RE, P - X0a);
@@ -350,6 +379,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
       issue_in2(r0 - 1, 0);
       issue_up(r0 - 1);
     }
+    __syncwarp();
     if (!wait_for(0, par0)) return;
     par0 ^= 1u;
     {
@@ -386,10 +416,13 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
                    reinterpret_cast<const float *>(sm + S::PS) + rr * RE, dcur + rr * RE, S::FB32 / 4,
                    reinterpret_cast<const double4 *>(sm + S::MY)[rr], o[rr], rr == H - 1 ? ly : nullptr, true);
       __syncwarp();
-      if (c < r1 && lane == 0) {
-        fence_proxy_async();
-        mbar_arrive_expect_tx(bar, IN_BYTES);
-        issue_in1(c + 1);
+      if (c < r1) {
+        if (elect_one()) {
+          fence_proxy_async();
+          mbar_arrive_expect_tx(bar, IN_BYTES);
+          issue_in1(c + 1);
+        }
+        __syncwarp();
       }
       if (c >= r0)
         if (!wait_for(1, par1)) return;
@@ -552,10 +585,13 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         }
         __syncwarp();
       }
-      if (c < r1 && lane == 0) {
-        fence_proxy_async();
-        issue_in2(c + 1, sl ^ 1);
-        if (c >= r0) issue_up(c);
+      if (c < r1) {
+        if (elect_one()) {
+          fence_proxy_async();
+          issue_in2(c + 1, sl ^ 1);
+          if (c >= r0) issue_up(c);
+        }
+        __syncwarp();
       }
       sl ^= 1;
       if (c < r1) {
@@ -630,65 +666,5 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     }
   }
 }
-
-template <int D>
-struct StripConfig {
-  template <int KIND>
-  using S = StripSmem<D, KIND>;
-  template <int KIND, int NB, bool IDENT>
-  static void launch_nb(dim3 grid, cudaStream_t s, const StageBatch<NB> &b, bool pdl) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(32 * S<KIND>::WPB);
-    cfg.dynamicSmemBytes = (size_t)S<KIND>::WPB * S<KIND>::BYTES;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, strip_kernel<D, KIND, NB, IDENT>, b);
-  }
-  template <int KIND>
-  static void launch(dim3 grid, cudaStream_t s, const StageBatch<1> &b, bool pdl) {
-    launch_nb<KIND, 1, false>(grid, s, b, pdl);
-  }
-  template <int KIND>
-  static void launch_ident(dim3 grid, cudaStream_t s, const StageBatch<1> &b, bool pdl) {
-    launch_nb<KIND, 1, true>(grid, s, b, pdl);
-  }
-  template <int KIND>
-  static void launch_batch(dim3 grid, cudaStream_t s, const StageBatch<kMaxGrids> &b, bool pdl) {
-    launch_nb<KIND, kMaxGrids, false>(grid, s, b, pdl);
-  }
-  template <int KIND>
-  static cudaError_t attr() {
-    const int bytes = S<KIND>::WPB * S<KIND>::BYTES;
-    cudaError_t e = cudaFuncSetAttribute(strip_kernel<D, KIND, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(strip_kernel<D, KIND, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(strip_kernel<D, KIND, kMaxGrids, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               bytes);
-    return e;
-  }
-  static cudaError_t prepare() {
-    cudaError_t e;
-    if ((e = attr<0>()) || (e = attr<1>()) || (e = attr<2>()) || (e = attr<3>()) || (e = attr<4>()) ||
-        (e = attr<5>()) || (e = attr<6>()))
-      return e;
-    return cudaSuccess;
-  }
-  static int blocks_per_sm() { return 1; }
-  static StageLauncher make() {
-    return StageLauncher{kStripCells, 1, 32 * S<1>::WPB, 1, 0, true, (size_t)S<1>::WPB * S<1>::BYTES, S<1>::RE, S<1>::H,
-                    {&launch<0>, &launch<1>, &launch<2>, &launch<3>, &launch<4>, &launch<5>, &launch<6>},
-                    {&launch_ident<0>, &launch_ident<1>, &launch_ident<2>, &launch_ident<3>, &launch_ident<4>,
-                     &launch_ident<5>, &launch_ident<6>},
-                    {&launch_batch<0>, &launch_batch<1>, &launch_batch<2>, &launch_batch<3>, &launch_batch<4>,
-                     &launch_batch<5>, &launch_batch<6>}, &prepare, &blocks_per_sm,
-                    {S<0>::WPB, S<1>::WPB, S<2>::WPB, S<3>::WPB, S<4>::WPB, S<5>::WPB, S<6>::WPB}};
-  }
-};
 
 }  // namespace mcv

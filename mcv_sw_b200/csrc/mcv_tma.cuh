@@ -21,8 +21,9 @@ namespace mcv {
 // Split precision: yu, yv, yp (FP64), phis32, du, dv, dp (FP32).
 // Strip form: yu, yv, yp, sqrtG of one panel (FP64), phis32, du, dv, dp (FP32),
 // met2 (8-byte pairs), the RK4 sums fU, fV, fP (FP32).
+// Strip form, FP64: the FP64 policy's eight, rsg, sgf, the RK base u0, v0, p0, the RK4 sums aU, aV, aP.
 struct TileMaps {
-  CUtensorMap f[12];
+  CUtensorMap f[16];
   int total;  // work items of the launch: tiles x 6 panels x active members
   int pad[15];
 };

@@ -9,7 +9,7 @@
 
 namespace mcv {
 
-StageLauncher strip_launcher_d3();  // stage_strip_mix.cu
+StageLauncher strip_launcher_d3_mix();  // stage_strip_d3_mix.cu
 
 const StageLauncher *stage_launchers_d3_mix(int *count) {
   static const StageLauncher table[] = {
@@ -21,7 +21,7 @@ const StageLauncher *stage_launchers_d3_mix(int *count) {
     StageConfig<3, 12, 12, 320, 2, true, 0, true>::make(),
     StageConfig<3, 12, 12, 320, 2, true, 2, true, 2>::make(),
     StageConfig<3, 12, 12, 320, 2, true, 3, true, 3>::make(),
-    strip_launcher_d3()};
+    strip_launcher_d3_mix()};
   *count = (int)(sizeof(table) / sizeof(table[0]));
   return table;
 }

@@ -9,7 +9,7 @@
 
 namespace mcv {
 
-StageLauncher strip_launcher_d4();  // stage_strip_mix.cu
+StageLauncher strip_launcher_d4_mix();  // stage_strip_d4_mix.cu
 
 const StageLauncher *stage_launchers_d4_mix(int *count) {
   static const StageLauncher table[] = {
@@ -20,7 +20,7 @@ const StageLauncher *stage_launchers_d4_mix(int *count) {
     StageConfig<4, 8, 8, 256, 2, true, 0, true>::make(),
     StageConfig<4, 8, 8, 320, 2, true, 0, true>::make(),
     StageConfig<4, 8, 8, 320, 2, true, 2, true, 3>::make(),
-    strip_launcher_d4()};
+    strip_launcher_d4_mix()};
   *count = (int)(sizeof(table) / sizeof(table[0]));
   return table;
 }

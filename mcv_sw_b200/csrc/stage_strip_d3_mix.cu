@@ -1,0 +1,10 @@
+// stage_strip_d3_mix.cu -- the strip form of the stage kernel for MCV3, split precision.
+// Compiled without FMA contraction: its fused operations are written out, so
+// that one grid and several grids in a launch give the same bits.
+#include "mcv_strip_table.cuh"
+
+namespace mcv {
+
+StageLauncher strip_launcher_d3_mix() { return StripConfig<3, true>::make(); }
+
+}  // namespace mcv
