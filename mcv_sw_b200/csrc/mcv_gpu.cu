@@ -596,7 +596,7 @@ void number_items(StageBatch<NB> &b, int n) {
 // two halo rows and its start).
 template <int NB>
 void cut_strips(StageBatch<NB> &b, int n, int warps) {
-  constexpr double kStart = 2.0;
+  constexpr double kStart = 2.3;
   int most = 1;
   for (int k = 0; k < n; ++k) {
     b.nsx[k] = (b.g[k].Nc + kStripCells - 1) / kStripCells;

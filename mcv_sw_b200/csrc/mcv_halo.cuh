@@ -154,16 +154,34 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
   // rotated to the sphere (covProjPlane2Sphere, projection_mod.F90:79-96).  A
   // point at an end of the line is a boundary point and takes its raw copy;
   // the FP64 form, whose boundary this kernel rewrites, reads no state there.
-  auto neighbour = [&](int hh, int kk, double &zq, double &mq, double &pq) {
+  // What does not change while the stage kernel runs comes first (fixed): the
+  // rotation and, split precision, Y.
+  struct Fixed {
+    double4 M;
+    double yu, yv, yp;
+  };
+  auto fixed = [&](int hh, int kk, Fixed &f) {
+    const int ks = L.rev ? n - 1 - kk : kk;
+    f.M = a.Mtab[((q * 4 + e2) * (H + 1) + hh) * n + ks];
+    if constexpr (MIXED) {
+      int si, sj;
+      strip_point(e2, hh, ks, n, si, sj);
+      const long long os = mb + q * g.plane + (long long)(sj + H) * g.P + (si + H);
+      f.yu = a.u[os];
+      f.yv = a.v[os];
+      f.yp = a.phi[os];
+    }
+  };
+  auto neighbour = [&](int hh, int kk, const Fixed &fx, double &zq, double &mq, double &pq) {
     const int ks = L.rev ? n - 1 - kk : kk;
     const bool isb = (ks == 0 || ks == n - 1);
     int si, sj;
     strip_point(e2, hh, ks, n, si, sj);
-    const double4 M = a.Mtab[((q * 4 + e2) * (H + 1) + hh) * n + ks];
+    const double4 M = fx.M;
     double su, sv, sp;
     if constexpr (MIXED) {
       const long long os = mb + q * g.plane + (long long)(sj + H) * g.P + (si + H);
-      const double yu = a.u[os], yv = a.v[os], yp = a.phi[os];
+      const double yu = fx.yu, yv = fx.yv, yp = fx.yp;
       float du, dv, dp;
       if (isb) {
         const float4 b = a.bnd32[bb + q * 4 * n + boundary_slot(si, sj, n)];
@@ -208,6 +226,19 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
       cc = a.gcoef[(h - 1) * n + k];
     }
   }
+  // the neighbour point this thread stages, and the rotations of a boundary point
+  static_assert(H * kHaloWin <= NT, "one staged point per thread");
+  const int lo = max(k0 - kHaloLead, 0);  // the window staged: [lo, lo + kHaloWin)
+  const int hs = (e2 <= 1) ? 1 + (int)threadIdx.x % H : 1 + (int)threadIdx.x / kHaloWin;
+  const int ts = (e2 <= 1) ? (int)threadIdx.x / H : (int)threadIdx.x % kHaloWin;
+  const bool stages = (int)threadIdx.x < H * kHaloWin && lo + ts <= n - 1;
+  Fixed fs;
+  if (stages) fixed(hs, lo + ts, fs);
+  double4 Mo{}, Mn{};
+  if (live && h == 0) {
+    Mo = a.Mtab[((p * 4 + e) * (H + 1) + 0) * n + k];
+    Mn = a.Mtab[((q * 4 + e2) * (H + 1) + 0) * n + (L.rev ? n - 1 - k : k)];
+  }
   // Launched with programmatic dependent launch, the blocks may be resident
   // before the stage kernel that writes the increments, boundary copies and
   // (FP64 form) the state has completed: everything above reads only what it
@@ -218,6 +249,8 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
   // kernel writes, the others wait for its completion
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+  // stage the neighbour's lines 1..H over the window
+  if (stages) neighbour(hs, lo + ts, fs, wz[hs - 1][ts], wm[hs - 1][ts], wp[hs - 1][ts]);
   // the boundary line (h = 0) needs no staged values
   bool store = live;
   double zw = 0., mw = 0., ph = 0.;
@@ -231,8 +264,6 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
       double ou, ov, op, nu, nv, np_;
       raw_boundary(p, oi, oj, ou, ov, op);
       raw_boundary(q, ni, nj, nu, nv, np_);
-      const double4 Mo = a.Mtab[((p * 4 + e) * (H + 1) + 0) * n + k];
-      const double4 Mn = a.Mtab[((q * 4 + e2) * (H + 1) + 0) * n + ks];
       zw = 0.5 * ((Mo.x * ou + Mo.z * ov) + (Mn.x * nu + Mn.z * nv));
       mw = 0.5 * ((Mo.y * ou + Mo.w * ov) + (Mn.y * nu + Mn.w * nv));
       ph = 0.5 * (op + np_);
@@ -261,14 +292,6 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
     }
   }
 
-  // stage the neighbour's lines 1..H over the window [lo, lo + kHaloWin)
-  const int lo = max(k0 - kHaloLead, 0);
-  for (int s = threadIdx.x; s < H * kHaloWin; s += NT) {
-    const int hh = (e2 <= 1) ? 1 + s % H : 1 + s / kHaloWin;
-    const int t = (e2 <= 1) ? s / H : s % kHaloWin;
-    const int kk = lo + t;
-    if (kk <= n - 1) neighbour(hh, kk, wz[hh - 1][t], wm[hh - 1][t], wp[hh - 1][t]);
-  }
   __syncthreads();
 
   if (live && h > 0) {
@@ -284,7 +307,9 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
         qm[m] = wm[h - 1][t];
         qp[m] = wp[h - 1][t];
       } else {
-        neighbour(h, kk, qz[m], qm[m], qp[m]);
+        Fixed f;
+        fixed(h, kk, f);
+        neighbour(h, kk, f, qz[m], qm[m], qp[m]);
       }
     }
     zw = ghost_interp<D>(qz, cc.x, cc.y, a);

@@ -747,6 +747,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
     panel = blockIdx.y;
     mem = IDENT ? (int)blockIdx.z : active_member(a.active, a.ident, (int)blockIdx.z);
     wait_prerequisite_grid();
+    // the halo kernel that follows may become resident (it waits for this grid's
+    // completion before reading what it writes)
+    allow_dependent_launch();
   }
   const int c0x = tx * CX, c0y = ty * CY;
   const int ncx = min(CX, g.Nc - c0x), ncy = min(CY, g.Nc - c0y);
