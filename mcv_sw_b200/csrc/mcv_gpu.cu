@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -589,41 +590,54 @@ void number_items(StageBatch<NB> &b, int n) {
   b.total = nin + ned;
 }
 
-// Strips of a strip-form launch over b's first n grids on `warps` resident
-// warps: every grid's columns of at most kStripCells cells are cut into
-// segments of about the same number of cell rows, as many as give the least
-// (passes over the warps) x (rows of a segment + what a segment pays for its
-// two halo rows and its start).
+// Divides the columns of a strip-form launch over b's first n grids between
+// `warps` resident warps: segments of about the same number of cell rows in every
+// column, as many as give the least (passes over the warps) x (rows + what a
+// strip pays for its start and halo rows); or one run per warp where that saves
+// 4% or more and runs are short (StageBatch, mcv_strip.cuh).
 template <int NB>
-void cut_strips(StageBatch<NB> &b, int n, int warps) {
-  constexpr double kStart = 2.3;
+int cut_strips(StageBatch<NB> &b, int n, int warps) {
+  constexpr double kStart = (double)kStripStart / kStripUnit;
+  constexpr long long kLongRun = 32;  // cell rows
+  long long units = 0, rows = 0;
   int most = 1;
   for (int k = 0; k < n; ++k) {
     b.nsx[k] = (b.g[k].Nc + kStripCells - 1) / kStripCells;
+    const long long columns = 6LL * b.slots[k] * b.nsx[k];
+    units += columns * (b.g[k].Nc * kStripUnit + kStripStart);
+    rows += columns * b.g[k].Nc;
     most = std::max(most, b.g[k].Nc);
   }
+  if (units > INT_MAX / 2) return fail(MCV_ERR_ARG, "too many cell rows for one launch");
   double best = 1e300;
-  int rows = 1;
-  for (int len = 1; len <= most; ++len) {
+  int len = 1;
+  for (int l = 1; l <= most; ++l) {
     long long strips = 0;
-    for (int k = 0; k < n; ++k) strips += 6LL * b.slots[k] * b.nsx[k] * ((b.g[k].Nc + len - 1) / len);
-    const double cost = (double)((strips + warps - 1) / warps) * (len + kStart);
+    for (int k = 0; k < n; ++k) strips += 6LL * b.slots[k] * b.nsx[k] * ((b.g[k].Nc + l - 1) / l);
+    const double cost = (double)((strips + warps - 1) / warps) * (l + kStart);
     if (cost < best) {
       best = cost;
-      rows = len;
+      len = l;
     }
   }
+  const long long run = (units + (long long)warps * kStripUnit - 1) / ((long long)warps * kStripUnit);  // cell rows, up
+  const bool runs = run <= kLongRun && (double)run + kStart < 0.96 * best;
   b.ngrids = n;
-  b.total = 0;
+  int at = 0;
   for (int k = 0; k < n; ++k) {
-    b.sy[k] = (b.g[k].Nc + rows - 1) / rows;
-    b.s0[k] = b.total;
-    b.total += 6 * b.slots[k] * b.nsx[k] * b.sy[k];
+    const int columns = 6 * b.slots[k] * b.nsx[k];
+    b.t0[k] = at;
+    b.sy[k] = runs ? 0 : (b.g[k].Nc + len - 1) / len;
+    at += runs ? columns * (b.g[k].Nc * kStripUnit + kStripStart) : columns * b.sy[k];
   }
-  b.s0[n] = b.total;
+  b.t0[n] = at;
+  b.total = runs ? (int)std::min<long long>(warps, rows) : at;
+  b.run_q = at / b.total;
+  b.run_r = at % b.total;
+  return MCV_OK;
 }
 
-// Blocks of a persistent launch over b's first n grids, whose work it numbers.
+// Blocks of a persistent launch over b's first n grids, whose work it numbers (0: error).
 template <int NB>
 int plan_persistent(StageBatch<NB> &b, int n, const StageLauncher &L, int kind, int resident) {
   const int wpb = L.strip[kind];
@@ -631,7 +645,7 @@ int plan_persistent(StageBatch<NB> &b, int n, const StageLauncher &L, int kind, 
     number_items(b, n);
     return std::max(1, std::min(b.total, resident));
   }
-  cut_strips(b, n, resident * wpb);
+  if (cut_strips(b, n, resident * wpb)) return 0;
   return std::max(1, std::min(b.total, resident));
 }
 
@@ -648,6 +662,7 @@ int launch_stage(mcv_handle *h, int cand, int s, int c) {
     return MCV_OK;
   }
   const int ctas = plan_persistent(b, 1, L, kind, h->bps[cand] * h->nsm);
+  if (!ctas) return MCV_ERR_ARG;
   launch(dim3(ctas), h->stream, b, true);
   return MCV_OK;
 }
@@ -1774,6 +1789,7 @@ int enqueue_group_stage(mcv_group *g, const std::vector<mcv_handle *> &act, cons
   for (size_t k = 0; k < act.size(); ++k)
     if (int rc = add_grid(b, (int)k, act[k], L, s, curs[k])) return rc;
   const int ctas = plan_persistent(b, (int)act.size(), L, stage_kind(act[0], s), g->bps * act[0]->nsm);
+  if (!ctas) return MCV_ERR_ARG;
   L.launch_batch[stage_kind(act[0], s)](dim3(ctas), g->stream, b, true);
   launch_halo_batch<kMaxGrids>(act.data(), curs.data(), (int)act.size(), s, g->stream);
   return MCV_OK;

@@ -95,6 +95,9 @@ struct StageArgs {
 constexpr int kMaxGrids = 4;
 // strip form: owned cells per strip, lanes 1..29 (lane 31 lends its first point to lane 30)
 constexpr int kStripCells = 29;
+// What a strip pays for its start and its two halo rows, in cell rows: 2.25
+// (measured: MCV4 Nc=256 stages fit (rows + 2.2) x 3.6 us split precision)
+constexpr int kStripUnit = 8, kStripStart = 18;
 template <int NB>
 struct StageBatch {
   TileMaps tm[NB];  // tensor maps of each grid's staged fields (TMA form)
@@ -106,9 +109,14 @@ struct StageBatch {
   int in0[NB + 1];  // first edge-free item of each grid
   int ed0[NB + 1];  // first edge item of each grid, counted from nin
   int slots[NB];    // active members of each grid
-  // strip form: columns of at most kStripCells cells, segments of cell rows and
-  // the first strip of each grid
-  int nsx[NB], sy[NB], s0[NB + 1];
+  // strip form: nsx columns of at most kStripCells cells across a panel.  Either
+  // (sy > 0) every column is cut into sy segments of cell rows, total strips in
+  // all, the first of a grid t0; or `total` runs of equal length share the columns
+  // of every grid laid end to end, kStripUnit units a cell row and kStripStart in
+  // front of each column, from unit t0 of a grid on: run id starts at
+  // id run_q + id run_r / total.
+  int nsx[NB], sy[NB], t0[NB + 1];
+  int run_q, run_r;
 };
 
 // ---------------------------------------------------------------------------

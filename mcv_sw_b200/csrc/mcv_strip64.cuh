@@ -99,16 +99,18 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
   bool waited = false;
   const int stride = gridDim.x * WPB;
 
-  // strips are dealt to the blocks in turn, so that few strips use every SM
-  for (int s = warp * gridDim.x + blockIdx.x; s < b.total; s += stride) {
-    int k = 0;
-#pragma unroll
-    for (int j = 1; j < NB; ++j)
-      if (j < b.ngrids && s >= b.s0[j]) k = j;
+  // runs are dealt to the blocks in turn, so that few of them use every SM
+  for (int id = warp * gridDim.x + blockIdx.x; id < b.total; id += stride) {
+  // (segments: run_q = 1, run_r = 0)
+  int x = id * b.run_q + (int)((long long)id * b.run_r / b.total);
+  const int xe = (id + 1) * b.run_q + (int)((long long)(id + 1) * b.run_r / b.total);
+  while (x < xe) {
+    int k;
+    Strip st;
+    if (!next_strip(b, id, x, xe, k, st)) continue;
     const GridDesc &g = b.g[k];
     const StageArgs &a = b.a[k];
     const TileMaps &tm = b.tm[k];
-    const Strip st = decode_strip(b, s, k);
     const int c0 = st.c0, w = st.w, r0 = st.r0, r1 = st.r1, panel = st.panel;
     const int mem = IDENT ? st.slot : active_member(a.active, a.ident, st.slot);
     const int X0 = c0 * H;  // padded index of lane 0's first point
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
     const long long pbase = (long long)panel * g.plane, fbase = (long long)mem * g.mstride + pbase;
     const int P = g.P;
     const double inc = a.inc * g.inv_dx, sfx = g.dx;  // tendencies come times dx
-    if (s + stride >= b.total) allow_dependent_launch();
+    if (id + stride >= b.total && x >= xe) allow_dependent_launch();
     if (!waited) {
       wait_prerequisite_grid();  // the halo kernel before
       waited = true;
@@ -460,6 +462,7 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
       }
       __syncwarp();
     }
+  }
   }
 }
 
