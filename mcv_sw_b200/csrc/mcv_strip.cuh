@@ -126,8 +126,12 @@ struct StripSmem {
   static constexpr int ARX = H * H * 32 * 20, ARB = (int)align128(ARX > FIRST_ROW ? ARX : FIRST_ROW);
   static constexpr int BAR = AR + ARB;
   static constexpr int BYTES = (int)align128(BAR + 16);
-  // warps per block: as many as shared memory (227 KB) and registers allow, one block per SM
-  static constexpr int WMAX = D == 3 ? 16 : 8;
+  // Warps per block, one block per SM: as many as registers (MCV4: 8) and shared
+  // memory (227 KB) allow.  MCV3 takes 12, not the 16 that fit: with registers and
+  // shared memory left over, blocks of the halo kernel become resident before the
+  // strips end, and a stage with its halo kernel takes 26 us at Nc=181 instead of
+  // 32, at no cost to large grids (64 members at Nc=128: 2.31 ms/step, was 2.40).
+  static constexpr int WMAX = D == 3 ? 12 : 8;
   static constexpr int WPB = 232448 / BYTES < WMAX ? 232448 / BYTES : WMAX;
   static_assert(H * 32 <= 128, "metric entries of the rows");
 };
@@ -453,6 +457,12 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
           fence_proxy_async();
           mbar_arrive_expect_tx(bar, IN_BYTES);
           issue_in1(c + 1);
+          if constexpr (S::ND == 2 || S::NY == 2) {
+            // issue_in2 loads these when their slot is free, shortly before they are read
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+              tma_prefetch_2d(&tm.f[S::ND == 2 ? 5 + f : f], X0a, frow + (c + 2) * H + 1);
+          }
         }
         __syncwarp();
       }
