@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel(const __grid_constant__
       bad = __syncthreads_or(!mbar_wait_bounded(bar, parity));
     }
     if (bad) {
-      if (threadIdx.x == 0) atomicExch(a.err, 1);
+      if (threadIdx.x == 0) *(volatile int *)a.err = 1;
       mbar_wait_bounded(bar, parity);  // the copies in flight land before the CTA exits
       return;
     }

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
       if (!__all_sync(ALL, ok)) {
         if (!ok) ok = mbar_wait_bounded(bar + i, parity);
         if (!__all_sync(ALL, ok)) {
-          if (lane == 0) atomicExch(a.err, 1);
+          if (lane == 0) *(volatile int *)a.err = 1;
           mbar_wait_bounded(bar, par0);
           mbar_wait_bounded(bar + 1, par1);
           return false;
