@@ -736,52 +736,95 @@ int enqueue_stage(mcv_handle *h, int s, int c, cudaEvent_t mid = nullptr) {
   return MCV_OK;
 }
 
-// Time every candidate shape on this grid with the first two stages of a step
-// (which leave the state alone) and the halo kernels after them, and keep the
-// fastest: the forms overlap the halo kernel to different extents, so the stage
-// kernel's time alone does not order them (MCV4 Nc=90, split precision: strips
-// 18.8 us a stage alone and 25.5 in a step, 8x8-cell tiles 19.4 and 21.8).
+// A step's first stages (which leave the state alone) and their halo kernels with
+// one candidate form, launched as in a step.
+int enqueue_trial(mcv_handle *h, int cand, int stages) {
+  for (int st = 0; st < stages; ++st) {
+    if (int rc = launch_stage(h, cand, st, h->cur)) return rc;
+    launch_halo(h, st, h->cur);
+  }
+  return MCV_OK;
+}
+
+// Small grids: the candidates' first stages in one graph, with event records
+// between them.  Plain launches would time the host, at about 9 us a stage for
+// every form: MCV3 Nc=32 FP64 took one of 30.8 us a step where another takes 28.8.
+int time_in_graph(mcv_handle *h, const std::vector<cudaEvent_t> &ev) {
+  MCV_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin trial capture");
+  int rc = MCV_OK;
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < h->ncands && !rc && e == cudaSuccess; ++i) {
+    rc = enqueue_trial(h, i, 1);  // warm-up
+    e = cudaEventRecordWithFlags(ev[2 * i], h->stream, cudaEventRecordExternal);
+    for (int r = 0; r < 3 && !rc; ++r) rc = enqueue_trial(h, i, 1);
+    if (e == cudaSuccess) e = cudaEventRecordWithFlags(ev[2 * i + 1], h->stream, cudaEventRecordExternal);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  cudaGraph_t graph = nullptr;
+  const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
+  cudaGraphExec_t exec = nullptr;
+  if (!rc && e == cudaSuccess) e = ce;
+  if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (exec) {
+    e = cudaGraphLaunch(exec, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaGraphExecDestroy(exec);
+  }
+  if (rc) return rc;
+  MCV_CUDA(e, "time stage kernels");
+  for (int i = 0; i < h->ncands; ++i) {
+    float ms = 0.f;
+    MCV_CUDA(cudaEventElapsedTime(&ms, ev[2 * i], ev[2 * i + 1]), "time stage kernels");
+    h->tune_ms[i] = ms / 3.f;  // per stage
+  }
+  return MCV_OK;
+}
+
+// Larger grids: one candidate after another, the strip form (the likely winner)
+// first; a form whose warm-up trial already takes a quarter longer than the best
+// is not timed further (MCV4 Nc=256 FP64, first step: 13.8 ms with all of them in full, 4.5 so).
+int time_in_turn(mcv_handle *h, const std::vector<cudaEvent_t> &ev) {
+  float best = 1e30f;
+  for (int i = h->ncands - 1; i >= 0; --i) {
+    float ms = 0.f;
+    for (int reps = 1; reps <= 2; ++reps) {
+      cudaEventRecord(ev[0], h->stream);
+      for (int r = 0; r < reps; ++r)
+        if (int rc = enqueue_trial(h, i, 2)) return rc;
+      cudaEventRecord(ev[1], h->stream);
+      MCV_CUDA(cudaEventSynchronize(ev[1]), "time stage kernels");
+      MCV_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]), "time stage kernels");
+      MCV_CUDA(cudaGetLastError(), "time stage kernels");
+      h->tune_ms[i] = ms / (2 * reps);  // per stage
+      if (h->tune_ms[i] > 1.25f * best) break;
+    }
+    best = std::min(best, h->tune_ms[i]);
+  }
+  return MCV_OK;
+}
+
+// Time the candidate shapes on this grid with the first two stages of a step and
+// the halo kernels after them, and keep the fastest: the forms overlap the halo
+// kernel to different extents, so the stage kernel's time alone does not order
+// them (MCV4 Nc=90, split precision: strips 18.8 us a stage alone and 25.5 in a
+// step, 8x8-cell tiles 19.4 and 21.8).
 int autotune(mcv_handle *h) {
   if (h->choice >= 0) return MCV_OK;
   h->tune_ms.assign(h->ncands, -1.f);
-  cudaEvent_t e0, e1;
-  MCV_CUDA(cudaEventCreate(&e0), "event");
-  MCV_CUDA(cudaEventCreate(&e1), "event");
-  float best = 1e30f;
-  int besti = 0;
+  std::vector<cudaEvent_t> ev(2 * h->ncands, nullptr);
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < h->ncands && e == cudaSuccess; ++i) {
-    // the step's first two stages and their halo kernels, launched as in a step
-    auto stages = [&]() {
-      for (int st = 0; st < 2; ++st) {
-        if (int rc = launch_stage(h, i, st, h->cur)) return rc;
-        launch_halo(h, st, h->cur);
-      }
-      return (int)MCV_OK;
-    };
-    int rc = stages();  // warm-up
-    cudaEventRecord(e0, h->stream);
-    for (int r = 0; r < 3 && !rc; ++r) rc = stages();
-    if (rc) {
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      return rc;
-    }
-    cudaEventRecord(e1, h->stream);
-    e = cudaEventSynchronize(e1);
-    float ms = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    h->tune_ms[i] = ms / 6.f;  // per stage
-    if (e == cudaSuccess && h->tune_ms[i] < best) {
-      best = h->tune_ms[i];
-      besti = i;
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (e != cudaSuccess) return cuda_fail(e, "autotune stage kernel");
-  h->choice = besti;
+  for (cudaEvent_t &x : ev)
+    if (e == cudaSuccess) e = cudaEventCreate(&x);
+  int rc = e == cudaSuccess ? MCV_OK : cuda_fail(e, "event");
+  // The line: a first step of MCV3 Nc=96 FP64 (0.22 M points) takes 1.02 ms with the
+  // trials in one graph and 1.25 with them in turn; 4 members of it 2.0 and 1.6.
+  const long long points = 6LL * h->g.np * h->g.np * h->n_active;
+  if (!rc) rc = points <= 262144 ? time_in_graph(h, ev) : time_in_turn(h, ev);
+  for (cudaEvent_t x : ev)
+    if (x) cudaEventDestroy(x);
+  if (rc) return rc;
+  h->choice = (int)(std::min_element(h->tune_ms.begin(), h->tune_ms.end()) - h->tune_ms.begin());
   return MCV_OK;
 }
 
