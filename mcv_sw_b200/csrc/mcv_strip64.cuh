@@ -170,16 +170,18 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
     };
     auto row_values = [&](const double *f, int fs, Row &o, double *cv, int cvst, double *ly) {
       const int at = rem + lane * H;
+      double p[8][H];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) lane_load<H>(f + x * fs + at, p[x]);
 #pragma unroll
       for (int i = 0; i < H; ++i) {
-        const double *p = f + at + i;
-        const double u = p[0], v = p[fs], ph = p[2 * fs], g11 = p[5 * fs], g12 = p[6 * fs], g22 = p[7 * fs];
+        const double u = p[0][i], v = p[1][i], ph = p[2][i], g11 = p[5][i], g12 = p[6][i], g22 = p[7][i];
         const double cu = __fma_rn(g12, v, g11 * u);  // cov2contrav, projection_mod.F90:138-148
         const double cw = __fma_rn(g22, v, g12 * u);
         o.u[i] = u;
         o.v[i] = v;
-        o.e[i] = __fma_rn(0.5, __fma_rn(cw, v, cu * u), ph + p[3 * fs]);  // E = phi + phi_s + K
-        o.pg[i] = ph * p[4 * fs];
+        o.e[i] = __fma_rn(0.5, __fma_rn(cw, v, cu * u), ph + p[3][i]);  // E = phi + phi_s + K
+        o.pg[i] = ph * p[4][i];
         o.cu[i] = cu;
         cv[i * cvst] = cw;
         if (i == 0) o.lx = fabs(cu) + sqrt(g11 * ph);
@@ -250,6 +252,8 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
 
       // ---- y sweep (:95-125) of the lane's columns: the fluxes at the bottom of cell c, which complete
       // rows (c - 1) H + 1 .. c H of cell c - 1; their tendencies (:127-131) and RK stage update
+      constexpr int NP = H == 2 ? 2 : 1;  // points updated at once
+      double t[H][3][NP], rsg[H][NP], sf[H][NP];
 #pragma unroll
       for (int i = 0; i < H; ++i) {
         double f[D], gE, gM, gU, lE, rE, lV, rV, b1, b2;
@@ -311,34 +315,50 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
         if (c >= r0) {
 #pragma unroll
           for (int rr = 0; rr < H; ++rr) {
-            const int at = rr * RE + rem + lane * H + i, pt = (rr * H + i) * 32;
+            const int pt = (rr * H + i) * 32;
             const double cu = ar[3 * PE + pt], cv = cvp[pt];
+            // MCV4 is updated point by point, MCV3 both points of the lane at once
+            constexpr int N = NP;
+            const int at = rr * RE + rem + lane * H + (N == 2 ? 0 : i);
             const double *rs = reinterpret_cast<const double *>(sm + S::RS) + at;
-            const double rsg = rs[0], sf = rs[FE];
-            double *out = reinterpret_cast<double *>(sm + S::OUT) + at;
-            const double ab = __fma_rn(sfx, sf, ar[2 * PE + pt] - yU[rr]);
+            if (N == 1 || i == 0) {
+              lane_load<N>(rs, rsg[rr]);
+              lane_load<N>(rs + FE, sf[rr]);
+            }
+            const int q = N == 2 ? i : 0;
+            const double ab = __fma_rn(sfx, sf[rr][q], ar[2 * PE + pt] - yU[rr]);
             const double fx = ar[pt], dx = ar[PE + pt];
-            // RK3: fx and dx already hold KU u - inc fx and KU phiG - inc dx
+            // RK3: the update without its base; fx and dx already hold KU u - inc fx and KU phiG - inc dx
             if constexpr (S::RK3) {
-              out[0] = __fma_rn(KB, out[0], __fma_rn(inc, ab * cv, fx));
-              out[FE] = __fma_rn(KB, out[FE], __fma_rn(-inc, __fma_rn(ab, cu, yE[rr]), KU * ar[4 * PE + pt]));
-              out[2 * FE] = __fma_rn(KB, out[2 * FE], rsg * __fma_rn(-inc, yM[rr], dx));
+              t[rr][0][q] = __fma_rn(inc, ab * cv, fx);
+              t[rr][1][q] = __fma_rn(-inc, __fma_rn(ab, cu, yE[rr]), KU * ar[4 * PE + pt]);
+              t[rr][2][q] = rsg[rr][q] * __fma_rn(-inc, yM[rr], dx);
             } else {
-              double t[3];
-              t[0] = __fma_rn(ab, cv, -fx);
-              t[1] = -__fma_rn(ab, cu, yE[rr]);
-              t[2] = -(dx + yM[rr]) * rsg;
+              t[rr][0][q] = __fma_rn(ab, cv, -fx);
+              t[rr][1][q] = -__fma_rn(ab, cu, yE[rr]);
+              t[rr][2][q] = -(dx + yM[rr]) * rsg[rr][q];
+            }
+            if (N == 2 && i == 0) continue;
 #pragma unroll
-              for (int x = 0; x < 3; ++x) {
-                double sum = t[x];
-                if constexpr (S::ACC_IN || S::ACC_OUT) {
-                  double *ac = reinterpret_cast<double *>(sm + S::ACC) + x * FE + at;
-                  if constexpr (KIND == RK4_S1) *ac = t[x];
-                  else if constexpr (S::ACC_OUT) *ac = __fma_rn(2., t[x], *ac);
-                  else sum = (*ac + t[x]) * (1. / 6.);
+            for (int x = 0; x < 3; ++x) {
+              double *out = reinterpret_cast<double *>(sm + S::OUT) + x * FE + at, base[N];
+              lane_load<N>(out, base);
+              if constexpr (S::ACC_IN || S::ACC_OUT) {
+                double *ac = reinterpret_cast<double *>(sm + S::ACC) + x * FE + at, s[N];
+                if constexpr (S::ACC_IN) lane_load<N>(ac, s);
+                if constexpr (KIND == RK4_S1) lane_store<N>(ac, t[rr][x]);
+                else {
+#pragma unroll
+                  for (int y = 0; y < N; ++y)
+                    if constexpr (S::ACC_OUT) s[y] = __fma_rn(2., t[rr][x][y], s[y]);
+                    else t[rr][x][y] = (s[y] + t[rr][x][y]) * (1. / 6.);
+                  if constexpr (S::ACC_OUT) lane_store<N>(ac, s);
                 }
-                out[x * FE] = __fma_rn(inc, sum, out[x * FE]);
               }
+#pragma unroll
+              for (int y = 0; y < N; ++y)
+                base[y] = S::RK3 ? __fma_rn(KB, base[y], t[rr][x][y]) : __fma_rn(inc, t[rr][x][y], base[y]);
+              lane_store<N>(out, base);
             }
           }
         }
