@@ -110,12 +110,13 @@ struct StageBatch {
   int ed0[NB + 1];  // first edge item of each grid, counted from nin
   int slots[NB];    // active members of each grid
   // strip form: nsx columns of at most kStripCells cells across a panel.  Either
-  // (sy > 0) every column is cut into sy segments of cell rows, total strips in
-  // all, the first of a grid t0; or `total` runs of equal length share the columns
+  // (sy > 0) the columns of the first pm1 panels (of all members) are cut into sy
+  // segments of cell rows, those of the others into sy2, total strips in all, the
+  // first of a grid t0; or `total` runs of equal length share the columns
   // of every grid laid end to end, kStripUnit units a cell row and kStripStart in
   // front of each column, from unit t0 of a grid on: run id starts at
   // id run_q + id run_r / total.
-  int nsx[NB], sy[NB], t0[NB + 1];
+  int nsx[NB], sy[NB], sy2[NB], pm1[NB], t0[NB + 1];
   int run_q, run_r;
 };
 

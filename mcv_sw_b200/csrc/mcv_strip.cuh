@@ -44,15 +44,13 @@ __device__ __forceinline__ bool elect_one() {
 
 // A strip: cells [c0, c0 + w) of cell rows [r0, r1) of one panel of one active
 // member.  A warp takes, one after the other,
-//  - segments of columns, all cut alike: neighbouring columns are worked on at
-//    the same rows at the same time, so that a row of a field is read as a whole
-//    (panels fastest: split precision's six panels share the metric planes); or
+//  - segments of columns, cut alike over many panels: neighbouring columns are
+//    worked on at the same rows at the same time, so that a row of a field is read
+//    as a whole (panels fastest: split precision's six panels share the metric
+//    planes); or
 //  - a run of the columns laid end to end: the end of a column and the beginning
 //    of another, so that no warp is left over.
-// Grids of many strips per warp take segments (MCV4 Nc=1024 RK4 in runs of 93
-// rows: 5.41 ms/step against 3.93), grids that segments divide badly runs (MCV4
-// Nc=256 FP64 RK3: 540 segments of 25 or 26 rows on 592 warps 0.301 ms/step, runs
-// of 23.4 rows 0.283).
+// Which, the host decides (cut_strips).
 struct Strip {
   int c0, w, r0, r1, panel, slot;
 };
@@ -76,11 +74,18 @@ __device__ __forceinline__ bool next_strip(const StageBatch<NB> &b, int id, int 
     if (j < b.ngrids && at >= b.t0[j]) k = j;
   const int Nc = b.g[k].Nc, nsx = b.nsx[k];
   if (segments) {
-    const int local = id - b.t0[k], per = 6 * b.slots[k];
+    int local = id - b.t0[k], pm = 0, per = b.pm1[k], sy = b.sy[k];
+    const int first = per * nsx * sy;
+    if (local >= first) {
+      local -= first;
+      pm = per;
+      per = 6 * b.slots[k] - per;
+      sy = b.sy2[k];
+    }
     const int q = local / per, seg = q / nsx;
-    strip_column(b, k, local - q * per, q - seg * nsx, t);
-    t.r0 = Nc * seg / b.sy[k];
-    t.r1 = Nc * (seg + 1) / b.sy[k];
+    strip_column(b, k, pm + local - q * per, q - seg * nsx, t);
+    t.r0 = Nc * seg / sy;
+    t.r1 = Nc * (seg + 1) / sy;
     x = xe;
     return true;
   }
