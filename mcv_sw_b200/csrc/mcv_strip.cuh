@@ -579,26 +579,25 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
           fy[H - 1] = slE + gE;
           dy[H - 1] = gM;
           dudy[H - 1] = gU;
-          // MCV4: the column's operands before its first result is stored, past which the compiler moves no
-          // load (RK4 step at Nc=512 934 -> 916 us; MCV3 has no registers left for it)
-          [[maybe_unused]] float4 xs[H];
-          [[maybe_unused]] float cvs[H], up[H][3];  // up: RK4 sum or (RK3 stage 2) d
+          float4 xs[H];
+          float cvs[H];
           [[maybe_unused]] float2 ms[H];
+          [[maybe_unused]] float as[H][3];
           if constexpr (H == 3) {
 #pragma unroll
             for (int rr = 0; rr < H; ++rr) {
-              const int at = rr * RE + rem + lane * H + i;
               xs[rr] = ar[(rr * H + i) * 32];
               cvs[rr] = arv[(rr * H + i) * 32];
-              ms[rr] = met[at];
+              ms[rr] = met[rr * RE + rem + lane * H + i];
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                if constexpr (S::ACC_IN) up[rr][f] = reinterpret_cast<const float *>(sm + S::ACC + f * S::FB32)[at];
-                if constexpr (KIND == RK3_S2)
-                  up[rr][f] = reinterpret_cast<const float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32)[at];
+                if constexpr (S::ACC_IN) as[rr][f] = reinterpret_cast<const float *>(sm + S::ACC + f * S::FB32)[rr * RE + rem + lane * H + i];
+                if constexpr (KIND == RK3_S2) as[rr][f] = reinterpret_cast<const float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32)[rr * RE + rem + lane * H + i];
               }
             }
           }
+          if (S::LAST && !S::DEFER && i == 0)  // the base has had the first column's fluxes to arrive
+            if (!wait_for(1, par1)) return;
 #pragma unroll
           for (int rr = 0; rr < H; ++rr) {
             const int at = rr * RE + rem + lane * H;
@@ -629,7 +628,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
               if constexpr (S::ACC_IN || S::ACC_OUT) {
                 float *pa = reinterpret_cast<float *>(sm + S::ACC + f * S::FB32) + at0;
                 float ac[N];
-                if constexpr (S::ACC_IN && H == 3) ac[0] = up[rr][f];
+                if constexpr (S::ACC_IN && H == 3) ac[0] = as[rr][f];
                 else if constexpr (S::ACC_IN) lane_load<N>(pa, ac);
                 if constexpr (KIND == RK4_S1) lane_store<N>(pa, sum);
                 else {
@@ -658,7 +657,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
               } else if constexpr (KIND == RK3_S2) {
                 float *pd = reinterpret_cast<float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32) + at0;
                 float d[N];
-                if constexpr (H == 3) d[0] = up[rr][f];
+                if constexpr (H == 3) d[0] = as[rr][f];
                 else lane_load<N>(pd, d);
 #pragma unroll
                 for (int q = 0; q < N; ++q) d[q] = fmaf(wt, sum[q], a.wd * d[q]);
