@@ -113,19 +113,12 @@ struct StripSmem {
   static constexpr bool ACC_IN = KIND == RK4_S2 || KIND == RK4_S3 || KIND == RK4_S4;        // ... the RK4 sum
   static constexpr bool ACC_OUT = KIND == RK4_S1 || KIND == RK4_S2 || KIND == RK4_S3;       // ... and writes it
   static constexpr int FB64 = (int)align128((size_t)H * RE * 8), FB32 = (int)align128((size_t)H * RE * 4);
-  // The update's results take the place of what it last read: RK3 stage 2's of d
-  // (two slots of d), the last stage's of Y; the others have an array of their own.
-  // The last stage reads the Y of a cell row twice, for the point values and one cell
-  // row later, from L2, as the update's base, in the same slot: a second slot left
-  // room for 6 (RK4) or 7 warps of MCV4 instead of 8 (Nc=512 RK4 stage 4 325 -> 245 us,
-  // the step 1017 -> 933; Nc=256 RK3 step 199 -> 190).  MCV4 holds the increments back
-  // until the whole y sweep is done (without that 256 us, 943): two warps on an SM
-  // quarter do not hide the base's copies.  Three of MCV3 do, and lose by it
-  // (16 members at Nc=128, stage 4 118 us and 124).
-  static constexpr bool DEFER = LAST && D == 4;
-  static constexpr int ND = FIRST ? 0 : (KIND == RK3_S2 || KIND == RK3_S3 ? 2 : 1);
+  // The update's results take the place of what it last read: the last stage's
+  // of Y + wd d (two slots of Y, the second filled by phase 0), RK3 stage 2's of d
+  // (two slots of d); the others have an array of their own.
+  static constexpr int NY = LAST ? 2 : 1, ND = FIRST ? 0 : (KIND == RK3_S2 ? 2 : 1);
   static constexpr int Y = 0, YS = 3 * FB64;               // Y_u, Y_v, Y_phi; a slot's size
-  static constexpr int SG = Y + YS;                        // sqrtG
+  static constexpr int SG = Y + NY * YS;                   // sqrtG
   static constexpr int PS = SG + FB64;                     // phi_s
   static constexpr int DU = PS + FB32, DS = 3 * FB32;      // d_u, d_v, d_phi
   static constexpr int OUT = DU + ND * DS;                 // results, where not in place
@@ -137,7 +130,7 @@ struct StripSmem {
   static constexpr int FIRST_ROW = (int)(4 * RE * 8 + 4 * RE * 4 + 32);  // the strip's first row, staged over AR
   static constexpr int ARX = H * H * 32 * 20, ARB = (int)align128(ARX > FIRST_ROW ? ARX : FIRST_ROW);
   static constexpr int BAR = AR + ARB;
-  static constexpr int BYTES = (int)align128(BAR + 24);
+  static constexpr int BYTES = (int)align128(BAR + 16);
   // Warps per block, one block per SM: as many as registers (MCV4: 8) and shared
   // memory (227 KB) allow.  MCV3 takes 12, not the 16 that fit: with registers and
   // shared memory left over, blocks of the halo kernel become resident before the
@@ -272,16 +265,14 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
   double *xt = reinterpret_cast<double *>(sm + S::XT);
   float4 *ar = reinterpret_cast<float4 *>(sm + S::AR) + lane;                    // x sweep: fx, dx, dvdx, cU
   float *arv = reinterpret_cast<float *>(sm + S::AR + H * H * 32 * 16) + lane;  // and cV of a point
-  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::BAR);  // [0] the input, [1] the update's operands, [2] its base (DEFER)
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::BAR);  // [0] the input, [1] the update's operands
   if (lane == 0) {
     mbar_init(bar, 1);
     mbar_init(bar + 1, 1);
-    mbar_init(bar + 2, 1);
     fence_mbar_init();
   }
   __syncwarp();
   uint32_t par0 = 0, par1 = 0;
-  [[maybe_unused]] uint32_t par2 = 0;
   bool waited = false;
   const int stride = gridDim.x * WPB;
 
@@ -323,14 +314,14 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     const int frow = (mem * 6 + panel) * g.np;
     constexpr uint32_t B64 = H * RE * 8, B32 = H * RE * 4;
     constexpr uint32_t IN_BYTES = 4 * B64 + B32 + (S::FIRST ? 0 : 3 * B32) + H * 32;
-    // what the update before leaves alone: sqrtG, phi_s, the metric entries, and Y and d unless
-    // they share their slots with it
+    // what the update before leaves alone: sqrtG, phi_s, the metric entries, and Y and d where
+    // their slots are free
     auto issue_in1 = [&](int c) {
       const int row = (c + 1) * H + 1;
       tma_load_2d(sm + S::SG, &tm.f[3], X0a, row, bar);
       tma_load_2d(sm + S::PS, &tm.f[4], X0a, frow + row, bar);
       bulk_load(sm + S::MY, a.met1d + row, H * 32, bar);
-      if constexpr (!S::LAST) {
+      if constexpr (S::NY == 1) {
 #pragma unroll
         for (int f = 0; f < 3; ++f) tma_load_2d(sm + S::Y + f * S::FB64, &tm.f[f], X0a, frow + row, bar);
       }
@@ -339,18 +330,19 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         for (int f = 0; f < 3; ++f) tma_load_2d(sm + S::DU + f * S::FB32, &tm.f[5 + f], X0a, frow + row, bar);
       }
     };
-    // what does: into the slot whose results have left
+    // what has two slots (RK3 stage 2: d; the last stage: Y), into the one whose results have left
     auto issue_in2 = [&](int c, int to) {
       const int row = (c + 1) * H + 1;
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         if constexpr (S::ND == 2)
           tma_load_2d(sm + S::DU + to * S::DS + f * S::FB32, &tm.f[5 + f], X0a, frow + row, bar);
-        if constexpr (S::LAST) tma_load_2d(sm + S::Y + f * S::FB64, &tm.f[f], X0a, frow + row, bar);
+        if constexpr (S::NY == 2)
+          tma_load_2d(sm + S::Y + to * S::YS + f * S::FB64, &tm.f[f], X0a, frow + row, bar);
       }
     };
     // operands of the update of cell row c's block
-    constexpr uint32_t UP_BYTES = B64 + (S::ACC_IN ? 3 * B32 : 0) + (S::LAST && !S::DEFER ? 3 * B64 : 0);
+    constexpr uint32_t UP_BYTES = B64 + (S::ACC_IN ? 3 * B32 : 0);
     auto issue_up = [&](int c) {
       const int row = (c + 1) * H + 1;
       mbar_arrive_expect_tx(bar + 1, UP_BYTES);
@@ -359,14 +351,6 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
 #pragma unroll
         for (int f = 0; f < 3; ++f) tma_load_2d(sm + S::ACC + f * S::FB32, &tm.f[9 + f], X0a, frow + row, bar + 1);
       }
-    };
-    // ... and the last stage's base, into the slots that the point values of the next have left
-    auto issue_base = [&](int c) {
-      const int row = (c + 1) * H + 1;
-      constexpr int B = S::DEFER ? 2 : 1;
-      if constexpr (S::DEFER) mbar_arrive_expect_tx(bar + B, 3 * B64);
-#pragma unroll
-      for (int f = 0; f < 3; ++f) tma_load_2d(sm + S::Y + f * S::FB64, &tm.f[f], X0a, frow + row, bar + B);
     };
     // Bounded wait for the copies of barrier i; false: give up (the copies in flight have landed or the
     // limit has run out twice).
@@ -378,7 +362,6 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
           if (lane == 0) *(volatile int *)a.err = 1;
           mbar_wait_bounded(bar, par0);
           mbar_wait_bounded(bar + 1, par1);
-          if constexpr (S::DEFER) mbar_wait_bounded(bar + 2, par2);
           return false;
         }
       }
@@ -388,8 +371,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     // pointwise quantities of one row (spatial_operators_mod.F90:58-61).  yf/sgf/psf/df: the row's
     // elements of lane 0 (Y fields fs apart, d fields ds apart); ly: the interface wave speeds in y
     // (for a row of interface points)
-    auto row_values = [&](const double *yf, int fs, const double *sgf, const float *psf, const float *df, int ds,
-                          const double4 my, StripRow<H> &o, float *ly) {
+    auto row_values = [&](double *yf, int fs, const double *sgf, const float *psf, const float *df, int ds,
+                          const double4 my, StripRow<H> &o, float *ly, bool base) {
       const double ty1 = __fma_rn(my.x, my.x, 1.), wy = (my.x * my.y) * r2;
       const int at = rem + lane * H;
       double y[3][H], sg[H], txs[H], cxs[H];
@@ -397,7 +380,18 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
         lane_load<H>(yf + f * fs + at, y[f]);
-        if constexpr (!S::FIRST) lane_load<H>(df + f * ds + at, d[f]);
+        if constexpr (!S::FIRST) {
+          lane_load<H>(df + f * ds + at, d[f]);
+          if constexpr (KIND == RK3_S3) {
+            // the update's base Y + wd d takes the place of these points' Y
+            if (base) {
+              double yb[H];
+#pragma unroll
+              for (int i = 0; i < H; ++i) yb[i] = __fma_rn((double)a.wd, (double)d[f][i], y[f][i]);
+              lane_store<H>(yf + f * fs + at, yb);
+            }
+          }
+        }
       }
       lane_load<H>(sgf + at, sg);
       lane_load<H>(psf + at, ps);
@@ -477,7 +471,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
       double *fr = reinterpret_cast<double *>(sm + S::AR);
       const float *fr32 = reinterpret_cast<const float *>(fr + 4 * RE);
       row_values(fr, RE, fr + 3 * RE, fr32, fr32 + RE, RE, *reinterpret_cast<const double4 *>(fr32 + 4 * RE), o,
-                 nullptr);
+                 nullptr, false);
 #pragma unroll
       for (int i = 0; i < H; ++i) {
         e0[i] = o.e[i];
@@ -498,34 +492,29 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
       // ---- rows c H + 1 .. c H + H (interior indices) of the lane's cell
       StripRow<H> o[H];
       float ly[H];
-      const double *ycur = reinterpret_cast<const double *>(sm + S::Y);
+      double *ycur = reinterpret_cast<double *>(sm + S::Y + (S::NY == 2 ? sl * S::YS : 0));
       const float *dcur = reinterpret_cast<const float *>(sm + S::DU + (S::ND == 2 ? sl * S::DS : 0));
 #pragma unroll
       for (int rr = 0; rr < H; ++rr)
         row_values(ycur + rr * RE, S::FB64 / 8, reinterpret_cast<const double *>(sm + S::SG) + rr * RE,
                    reinterpret_cast<const float *>(sm + S::PS) + rr * RE, dcur + rr * RE, S::FB32 / 4,
-                   reinterpret_cast<const double4 *>(sm + S::MY)[rr], o[rr], rr == H - 1 ? ly : nullptr);
+                   reinterpret_cast<const double4 *>(sm + S::MY)[rr], o[rr], rr == H - 1 ? ly : nullptr, true);
       __syncwarp();
-      if (S::LAST || c < r1) {
+      if (c < r1) {
         if (elect_one()) {
           fence_proxy_async();
-          if constexpr (S::LAST) {
-            if (c >= r0) issue_base(c - 1);
-          }
-          if (c < r1) {
-            mbar_arrive_expect_tx(bar, IN_BYTES);
-            issue_in1(c + 1);
+          mbar_arrive_expect_tx(bar, IN_BYTES);
+          issue_in1(c + 1);
+          if constexpr (S::ND == 2 || S::NY == 2) {
             // issue_in2 loads these when their slot is free, shortly before they are read
 #pragma unroll
-            for (int f = 0; f < 3; ++f) {
-              if constexpr (S::ND == 2) tma_prefetch_2d(&tm.f[5 + f], X0a, frow + (c + 2) * H + 1);
-              if constexpr (S::LAST) tma_prefetch_2d(&tm.f[f], X0a, frow + (c + 2) * H + 1);
-            }
+            for (int f = 0; f < 3; ++f)
+              tma_prefetch_2d(&tm.f[S::ND == 2 ? 5 + f : f], X0a, frow + (c + 2) * H + 1);
           }
         }
         __syncwarp();
       }
-      if ((!S::LAST || S::DEFER) && c >= r0)
+      if (c >= r0)
         if (!wait_for(1, par1)) return;
 
       // ---- y sweep (:95-125) of the lane's columns: the fluxes at the bottom of
@@ -579,8 +568,6 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
           fy[H - 1] = slE + gE;
           dy[H - 1] = gM;
           dudy[H - 1] = gU;
-          if (S::LAST && !S::DEFER && i == 0)  // the base has had the first column's fluxes to arrive
-            if (!wait_for(1, par1)) return;
 #pragma unroll
           for (int rr = 0; rr < H; ++rr) {
             const int at = rr * RE + rem + lane * H;
@@ -621,20 +608,12 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
                   if constexpr (S::ACC_OUT) lane_store<N>(pa, ac);
                 }
               }
-              if constexpr (S::DEFER) {
-                tt[rr][f][i] = wt * sum[0];
-              } else if constexpr (S::LAST) {
-                double *py = reinterpret_cast<double *>(sm + S::Y + f * S::FB64) + at0;
+              if constexpr (S::LAST) {
+                double *py = reinterpret_cast<double *>(sm + S::Y + (sl ^ 1) * S::YS + f * S::FB64) + at0;
                 double y[N];
                 lane_load<N>(py, y);
-                [[maybe_unused]] float d[N];
-                if constexpr (KIND == RK3_S3)
-                  lane_load<N>(reinterpret_cast<const float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32) + at0, d);
 #pragma unroll
-                for (int q = 0; q < N; ++q) {
-                  if constexpr (KIND == RK3_S3) y[q] = __fma_rn((double)a.wd, (double)d[q], y[q]);
-                  y[q] = y[q] + (double)(wt * sum[q]);
-                }
+                for (int q = 0; q < N; ++q) y[q] = y[q] + (double)(wt * sum[q]);
                 lane_store<N>(py, y);
               } else if constexpr (KIND == RK3_S2) {
                 float *pd = reinterpret_cast<float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32) + at0;
@@ -650,8 +629,6 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
                 lane_store<N>(reinterpret_cast<float *>(sm + S::OUT + f * S::FB32) + at0, r);
               }
             }
-            if constexpr (S::DEFER)  // in the place of the sweep's results
-              ar[(rr * H + i) * 32] = make_float4(tt[rr][0][i], tt[rr][1][i], tt[rr][2][i], 0.f);
           }
         }
         interior_chord<D>(gE, e1, e2, bE1[i], bE2[i]);
@@ -675,37 +652,6 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         cv0[i] = o[H - 1].cv[i];
       }
 
-      if constexpr (S::DEFER) {
-        if (c >= r0) {
-          if (!wait_for(2, par2)) return;
-          par2 ^= 1u;
-#pragma unroll
-          for (int rr = 0; rr < H; ++rr) {
-            const int at = rr * RE + rem + lane * H;
-            double *py = reinterpret_cast<double *>(sm + S::Y) + at;
-            const float *pd = reinterpret_cast<const float *>(sm + S::DU + (sl ^ 1) * S::DS) + at;
-            float4 inc[H];
-            double y[3][H];
-            [[maybe_unused]] float d[3][H];
-#pragma unroll
-            for (int i = 0; i < H; ++i) inc[i] = ar[(rr * H + i) * 32];
-#pragma unroll
-            for (int f = 0; f < 3; ++f) {
-              lane_load<H>(py + f * (S::FB64 / 8), y[f]);
-              if constexpr (KIND == RK3_S3) lane_load<H>(pd + f * (S::FB32 / 4), d[f]);
-            }
-#pragma unroll
-            for (int f = 0; f < 3; ++f) {
-#pragma unroll
-              for (int i = 0; i < H; ++i) {
-                if constexpr (KIND == RK3_S3) y[f][i] = __fma_rn((double)a.wd, (double)d[f][i], y[f][i]);
-                y[f][i] += (double)(f == 0 ? inc[i].x : f == 1 ? inc[i].y : inc[i].z);
-              }
-              lane_store<H>(py + f * (S::FB64 / 8), y[f]);
-            }
-          }
-        }
-      }
       if (c >= r0) {
         par1 ^= 1u;
         // ---- store the finished rows, one point per lane
@@ -714,7 +660,7 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         using Out = std::conditional_t<S::LAST, double, float>;
         constexpr int FB = S::LAST ? S::FB64 : S::FB32;
         const Out *res = reinterpret_cast<const Out *>(
-            sm + (S::LAST ? S::Y : KIND == RK3_S2 ? S::DU + (sl ^ 1) * S::DS : S::OUT));
+            sm + (S::LAST ? S::Y + (sl ^ 1) * S::YS : KIND == RK3_S2 ? S::DU + (sl ^ 1) * S::DS : S::OUT));
         for (int rr = lo; rr < hi; ++rr) {
           const int gj = (c - 1) * H + 1 + rr;  // 0-based interior row
           const long long ro = fbase + (long long)(gj + H) * P + (X0 + H) + lane;
