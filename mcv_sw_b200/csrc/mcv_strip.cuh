@@ -568,17 +568,37 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
           fy[H - 1] = slE + gE;
           dy[H - 1] = gM;
           dudy[H - 1] = gU;
+          // MCV4: the column's operands before its first result is stored, past which the compiler moves no
+          // load (RK4 step at Nc=512 1016 -> 943 us, RK3 at Nc=256 199 -> 192; MCV3 has no registers for it)
+          [[maybe_unused]] float4 xs[H];
+          [[maybe_unused]] float cvs[H], up[H][3];  // up: RK4 sum or (RK3 stage 2) d
+          [[maybe_unused]] float2 ms[H];
+          if constexpr (H == 3) {
+#pragma unroll
+            for (int rr = 0; rr < H; ++rr) {
+              const int at = rr * RE + rem + lane * H + i;
+              xs[rr] = ar[(rr * H + i) * 32];
+              cvs[rr] = arv[(rr * H + i) * 32];
+              ms[rr] = met[at];
+#pragma unroll
+              for (int f = 0; f < 3; ++f) {
+                if constexpr (S::ACC_IN) up[rr][f] = reinterpret_cast<const float *>(sm + S::ACC + f * S::FB32)[at];
+                if constexpr (KIND == RK3_S2)
+                  up[rr][f] = reinterpret_cast<const float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32)[at];
+              }
+            }
+          }
 #pragma unroll
           for (int rr = 0; rr < H; ++rr) {
             const int at = rr * RE + rem + lane * H;
-            const float4 x = ar[(rr * H + i) * 32];  // fx, dx, dvdx, cU
-            const float cv = arv[(rr * H + i) * 32];
+            const float4 x = H == 3 ? xs[rr] : ar[(rr * H + i) * 32];  // fx, dx, dvdx, cU
+            const float cv = H == 3 ? cvs[rr] : arv[(rr * H + i) * 32];
             float2 m;  // 1/sqrtG, sqrtG f
             if constexpr (H == 2) {
               if (i == 0) met2[rr] = *reinterpret_cast<const float4 *>(met + at);
               m = i == 0 ? make_float2(met2[rr].x, met2[rr].y) : make_float2(met2[rr].z, met2[rr].w);
             } else {
-              m = met[at + i];
+              m = ms[rr];
             }
             // sqrtG (vort + f) = (dvdx - dudy) + sqrtG f
             const float ab = fmaf(fdx, m.y, x.z - dudy[rr]);
@@ -598,7 +618,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
               if constexpr (S::ACC_IN || S::ACC_OUT) {
                 float *pa = reinterpret_cast<float *>(sm + S::ACC + f * S::FB32) + at0;
                 float ac[N];
-                if constexpr (S::ACC_IN) lane_load<N>(pa, ac);
+                if constexpr (S::ACC_IN && H == 3) ac[0] = up[rr][f];
+                else if constexpr (S::ACC_IN) lane_load<N>(pa, ac);
                 if constexpr (KIND == RK4_S1) lane_store<N>(pa, sum);
                 else {
 #pragma unroll
@@ -618,7 +639,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
               } else if constexpr (KIND == RK3_S2) {
                 float *pd = reinterpret_cast<float *>(sm + S::DU + (sl ^ 1) * S::DS + f * S::FB32) + at0;
                 float d[N];
-                lane_load<N>(pd, d);
+                if constexpr (H == 3) d[0] = up[rr][f];
+                else lane_load<N>(pd, d);
 #pragma unroll
                 for (int q = 0; q < N; ++q) d[q] = fmaf(wt, sum[q], a.wd * d[q]);
                 lane_store<N>(pd, d);
