@@ -401,8 +401,8 @@ class Stepper:
         return list(st)[:nst], ha.value
 
     def tuning(self):
-        """Autotuner record: list of ((cells_x, cells_y, threads, walk, ctas_per_sm, tma), ms per launch)
-        and the chosen index."""
+        """Autotuner record: list of ((cells_x, cells_y, threads, walk, ctas_per_sm, persistent), ms per
+        stage with its halo kernel) and the chosen index; the last is the strip form."""
         n, ch = ctypes.c_int(), ctypes.c_int()
         shapes = (ctypes.c_int * 96)()
         ms = (ctypes.c_float * 16)()
