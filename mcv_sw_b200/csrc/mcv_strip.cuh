@@ -42,6 +42,15 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// Before copies of an elected lane overwrite shared memory that the warp has used:
+// every lane orders its own reads and writes before later ones of the async proxy
+// (the fence acts on the accesses of the thread that executes it), then the warp
+// meets.  One instruction for the warp, as the elected lane's alone would be.
+__device__ __forceinline__ void hand_to_copies() {
+  fence_proxy_async();
+  __syncwarp();
+}
+
 // A strip: cells [c0, c0 + w) of cell rows [r0, r1) of one panel of one active
 // member.  A warp takes, one after the other,
 //  - segments of columns, cut alike over many panels: neighbouring columns are
@@ -441,8 +450,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
     float bE1[H], bE2[H], bM1[H], bM2[H], bU1[H], bU2[H];
 
     int sl = 0;  // the slot of the current cell row, where there are two
+    hand_to_copies();
     if (elect_one()) {
-      fence_proxy_async();
       // the first row of the lower halo cell, then its block
       const int row = r0 * H, nel = min(RE, P - X0a);
       const long long o = fbase + (long long)row * P + X0a, om = (long long)row * P + X0a;
@@ -499,10 +508,9 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
         row_values(ycur + rr * RE, S::FB64 / 8, reinterpret_cast<const double *>(sm + S::SG) + rr * RE,
                    reinterpret_cast<const float *>(sm + S::PS) + rr * RE, dcur + rr * RE, S::FB32 / 4,
                    reinterpret_cast<const double4 *>(sm + S::MY)[rr], o[rr], rr == H - 1 ? ly : nullptr, true);
-      __syncwarp();
+      hand_to_copies();
       if (c < r1) {
         if (elect_one()) {
-          fence_proxy_async();
           mbar_arrive_expect_tx(bar, IN_BYTES);
           issue_in1(c + 1);
           if constexpr (S::ND == 2 || S::NY == 2) {
@@ -727,11 +735,10 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
             }
           }
         }
-        __syncwarp();
       }
       if (c < r1) {
+        hand_to_copies();
         if (elect_one()) {
-          fence_proxy_async();
           issue_in2(c + 1, sl ^ 1);
           if (c >= r0) issue_up(c);
         }

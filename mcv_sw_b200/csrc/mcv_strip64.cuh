@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
     double e0[H], u0[H], v0[H], q0[H], m0[H], lam0[H], sE[H], sM[H], rU[H];
     double bE1[H], bE2[H], bM1[H], bM2[H], bU1[H], bU2[H];
 
+    hand_to_copies();
     if (elect_one()) {
-      fence_proxy_async();
       // the first row of the lower halo cell, then its block
       const int row = r0 * H, nel = min(RE, P - X0a);
       const long long o = (long long)row * P + X0a;
@@ -238,10 +238,9 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
 #pragma unroll
       for (int rr = 0; rr < H; ++rr)
         row_values(in + rr * RE, FE, o[rr], cvc + rr * H * 32, 32, rr == H - 1 ? ly : nullptr);
-      __syncwarp();
+      hand_to_copies();
       if (c < r1) {
         if (elect_one()) {
-          fence_proxy_async();
           mbar_arrive_expect_tx(bar, 8 * BB);
           issue_in(c + 1);
         }
@@ -406,10 +405,9 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
             }
           }
         }
-        __syncwarp();
         if (c < r1) {
+          hand_to_copies();
           if (elect_one()) {
-            fence_proxy_async();
             issue_up(c);
           }
           __syncwarp();
