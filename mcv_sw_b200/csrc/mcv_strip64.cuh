@@ -164,7 +164,8 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
 
     // pointwise quantities of one staged row (fields fs apart; spatial_operators_mod.F90:58-61), the
     // interface wave speeds |c| + sqrt(G^ii phi) (:248-280) in x at the cell's first point and, for a row
-    // of interface points, in y (with the sign of cV)
+    // of interface points, in y (the sign bit says cV < 0, which a wind of -0 is not and a speed that is
+    // not a number does not hide)
     struct Row {
       double e[H], u[H], v[H], pg[H], cu[H], lx;
     };
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
         o.cu[i] = cu;
         cv[i * cvst] = cw;
         if (i == 0) o.lx = fabs(cu) + sqrt(g11 * ph);
-        if (ly) ly[i] = copysign(fabs(cw) + sqrt(g22 * ph), cw);
+        if (ly) ly[i] = copysign(fabs(cw) + sqrt(g22 * ph), cw < 0. ? -1. : 1.);
       }
     };
 
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
 #pragma unroll
         for (int m = 1; m < D; ++m) f[m] = o[m - 1].u[i];
         lE = end_left<D>(f);
-        gU = lam0[i] < 0. ? lE : rU[i];
+        gU = __double2hiint(lam0[i]) < 0 ? lE : rU[i];
         rU[i] = end_right<D>(f);
         u0[i] = f[H];
         yU[0] = interior64_end1<D>(bU1[i], gU);
