@@ -224,11 +224,13 @@ Layout make_layout(const GridDesc &g, int H, int scheme, int precision, int memb
     L.sgm = take(sizeof(double) * (size_t)g.plane);
     L.met2 = take(sizeof(float2) * 2 * (size_t)g.plane);
     L.phibar = take(sizeof(double) * members);
-    // 96-byte linear-reference records for the most tiles any candidate shape makes
+    // 96-byte linear-reference records for the most tiles any TMA tile form makes
+    // (the direct tiles keep theirs in shared memory, the strips have none)
     int ncand = 0, most = 0;
     const StageLauncher *cands = stage_launchers(H + 1, true, &ncand);
     for (int c = 0; c < ncand; ++c)
-      most = std::max(most, ((g.Nc + cands[c].CX - 1) / cands[c].CX) * ((g.Nc + cands[c].CY - 1) / cands[c].CY));
+      if (cands[c].tma && !cands[c].strip[0])
+        most = std::max(most, ((g.Nc + cands[c].CX - 1) / cands[c].CX) * ((g.Nc + cands[c].CY - 1) / cands[c].CY));
     L.prec = take((size_t)96 * 6 * most * members);
   }
   for (int k = 0; k < 5; ++k) L.metric[k] = take(plane6);
