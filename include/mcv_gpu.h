@@ -121,7 +121,10 @@ int mcv_step(mcv_handle *h, int nsteps);
 
 /* Queue nsteps on the handle's stream and return without waiting. */
 int mcv_step_async(mcv_handle *h, int nsteps);
-/* Wait for the work queued on the handle's stream. */
+/* Wait for the work queued on the handle's stream.  Fails if a stage kernel gave
+ * up on copies that did not arrive in time (mcv_selftest_wait), and from then on
+ * until the geometry is set again (mcv_set_geometry or
+ * mcv_set_geometry_equiangular); the states must be set again, too. */
 int mcv_sync(mcv_handle *h);
 /* MCV_OK if all work queued on the handle has finished, MCV_BUSY if some is
  * still running; never waits. */

@@ -383,6 +383,12 @@ int download_state(mcv_handle *h, double *const *dst, double *const *src) {
   return MCV_OK;
 }
 
+// The stage kernels' error flag, once their work has ended.
+int check_late(const mcv_handle *h) {
+  if (*h->late) return fail(MCV_ERR_CUDA, "stage kernel: a staged tile's copies did not arrive in time");
+  return MCV_OK;
+}
+
 int num_stages(const mcv_handle *h) { return h->scheme == MCV_RK3_TVD ? 3 : 4; }
 
 // Stage kind of stage s of the handle's scheme.
@@ -872,6 +878,7 @@ int autotune(mcv_handle *h) {
   if (!rc) rc = points <= 262144 ? time_in_graph(h, ev) : time_in_turn(h, ev);
   for (cudaEvent_t x : ev)
     if (x) cudaEventDestroy(x);
+  if (!rc) rc = check_late(h);  // a form that gave up was timed for work it did not do
   if (rc) return rc;
   h->choice = (int)(std::min_element(h->tune_ms.begin(), h->tune_ms.end()) - h->tune_ms.begin());
   return MCV_OK;
@@ -1218,6 +1225,7 @@ extern "C" int mcv_set_geometry(mcv_handle *h, const double *sqrtG, const double
              "upload metric table");
   if ((rc = build_metric_planes(h))) return rc;
   MCV_CUDA(cudaStreamSynchronize(h->stream), "geometry upload");
+  *h->late = 0;  // the handle starts over
   h->sqrtG_host.assign(sqrtG, sqrtG + NP);
   h->geometry_set = true;
   return MCV_OK;
@@ -1260,6 +1268,7 @@ extern "C" int mcv_set_geometry_equiangular(mcv_handle *h) {
   h->sqrtG_host.resize(NP);
   if (int rc = download_padded(h, h->sqrtG_host.data(), h->sqrtG)) return rc;
   MCV_CUDA(cudaStreamSynchronize(h->stream), "device geometry");
+  *h->late = 0;  // the handle starts over
   if (bad) return fail(MCV_ERR_ARG, "ghost cell location error");
   h->geometry_set = true;
   return MCV_OK;
@@ -1465,8 +1474,7 @@ extern "C" int mcv_step_async(mcv_handle *h, int nsteps) {
 extern "C" int mcv_sync(mcv_handle *h) {
   if (!h) return fail(MCV_ERR_ARG, "handle is NULL");
   MCV_CUDA(cudaStreamSynchronize(h->stream), "step");
-  if (*h->late) return fail(MCV_ERR_CUDA, "stage kernel: a staged tile's copies did not arrive in time");
-  return MCV_OK;
+  return check_late(h);
 }
 
 namespace {
@@ -1517,6 +1525,21 @@ extern "C" int mcv_selftest_wait(int complete, double limit_ms, int *timed_out, 
   if (e != cudaSuccess) return cuda_fail(e, "wait self-test");
   *timed_out = o.timed_out;
   *elapsed_ms = (double)o.elapsed_ns * 1e-6;
+  return MCV_OK;
+}
+
+namespace {
+
+__global__ void raise_late_kernel(int *late) { *(volatile int *)late = 1; }
+
+}  // namespace
+
+// For the tests: raises the handle's late-copies flag from the device, as a stage
+// kernel does that gives up.
+extern "C" int mcv_selftest_late(mcv_handle *h) {
+  if (!h) return fail(MCV_ERR_ARG, "handle is NULL");
+  raise_late_kernel<<<1, 1, 0, h->stream>>>(h->late_dev);
+  MCV_CUDA(cudaGetLastError(), "raise the late-copies flag");
   return MCV_OK;
 }
 
