@@ -161,7 +161,10 @@ int mcv_selftest_wait(int complete, double limit_ms, int *timed_out, double *ela
  * them (each grid with its own geometry, dt and state buffers), followed by
  * each grid's halo kernel; a group step is one CUDA graph.  tile: the
  * stage-kernel candidate of the launch (mcv_tuning's index of a persistent
- * TMA form), or -1 for the first handle's choice.  Each handle's result is
+ * form: TMA tiles or strips), or -1 for the first handle's choice; if that is
+ * the autotuner's and a direct tile, split precision takes the fastest
+ * persistent form of its record (FP64, and a direct tile set by
+ * mcv_select_tile, are refused).  Each handle's result is
  * bit for bit that of the handle stepped alone on the same candidate.  The
  * handles keep working alone as well: the group orders its work after what
  * is queued on their streams, and their later work after the group's.

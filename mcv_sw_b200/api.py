@@ -441,7 +441,8 @@ class Group:
     """Several Steppers (one order, precision and scheme; any Nc, dt, members)
     advanced together, one batched stage-kernel launch per RK stage
     (mcv_group_*).  tile: the candidate index of the launch, or -1 for the
-    first stepper's choice."""
+    first stepper's choice (split precision, where that is a direct tile: the
+    fastest persistent form it timed)."""
 
     def __init__(self, steppers, tile=-1):
         self.steppers = list(steppers)

@@ -161,6 +161,7 @@ struct mcv_handle {
   // stage kernel chosen by the autotuner
   const StageLauncher *cands = nullptr;
   int ncands = 0, choice = -1;
+  bool tuned = false;  // the choice is the autotuner's, not mcv_select_tile's
   std::vector<float> tune_ms;
   cudaGraphExec_t graph_exec[2]{};
 };
@@ -881,6 +882,7 @@ int autotune(mcv_handle *h) {
   if (!rc) rc = check_late(h);  // a form that gave up was timed for work it did not do
   if (rc) return rc;
   h->choice = (int)(std::min_element(h->tune_ms.begin(), h->tune_ms.end()) - h->tune_ms.begin());
+  h->tuned = true;
   return MCV_OK;
 }
 
@@ -1930,6 +1932,7 @@ extern "C" int mcv_select_tile(mcv_handle *h, int index) {
       h->graph_exec[c] = nullptr;
     }
   h->choice = index;  // -1: autotune again before the next step
+  h->tuned = false;
   if (index >= 0 && (int)h->tune_ms.size() != h->ncands) h->tune_ms.assign(h->ncands, -1.f);
   return MCV_OK;
 }
@@ -2048,6 +2051,24 @@ int prepare_group(mcv_group *g, std::vector<mcv_handle *> &act, int &flip) {
 
 }  // namespace
 
+namespace {
+
+// The form of a group that names none: its first handle's choice.  Where the
+// autotuner chose a direct tile, which runs one grid only, split precision takes the
+// fastest persistent form it timed: on small grids the two are close (MCV3 Nc=32 RK4
+// 34.9 and 35.6 us a step, Nc=48 39.0 both), and one launch for several grids saves
+// more.  FP64's persistent tiles are slower than its direct ones (MCV3 Nc=32 28.8 and
+// 34.9), so its grids step alone.
+int group_form(const mcv_handle *h) {
+  if (!h->mixed || !h->tuned || h->cands[h->choice].tma) return h->choice;
+  int best = -1;
+  for (int i = 0; i < h->ncands; ++i)
+    if (h->cands[i].tma && h->tune_ms[i] >= 0.f && (best < 0 || h->tune_ms[i] < h->tune_ms[best])) best = i;
+  return best;
+}
+
+}  // namespace
+
 extern "C" int mcv_group_create(mcv_handle *const *handles, int count, int tile, mcv_group **out) {
   if (!out) return fail(MCV_ERR_ARG, "out is NULL");
   *out = nullptr;
@@ -2061,9 +2082,9 @@ extern "C" int mcv_group_create(mcv_handle *const *handles, int count, int tile,
         h->scheme != handles[0]->scheme || h->device != handles[0]->device)
       return fail(MCV_ERR_ARG, "the handles of a group share order, precision, scheme and device");
   }
-  const int cand = tile >= 0 ? tile : handles[0]->choice;
+  const int cand = tile >= 0 ? tile : group_form(handles[0]);
   if (cand < 0 || cand >= handles[0]->ncands || !handles[0]->cands[cand].tma)
-    return fail(MCV_ERR_ARG, "the group's stage-kernel candidate must be a persistent TMA form (mcv_tuning)");
+    return fail(MCV_ERR_ARG, "the group's stage-kernel candidate must be a persistent form: TMA tiles or strips (mcv_tuning)");
   mcv_group *g = new mcv_group();
   g->hs.assign(handles, handles + count);
   g->cand = cand;

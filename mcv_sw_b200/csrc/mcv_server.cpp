@@ -520,7 +520,7 @@ extern "C" int mcv_server_poll(mcv_server *s, long long *ids, int max_ids, int *
       } else if (mcv_group_create(hs.data(), (int)hs.size(), s->tile, &grp) == MCV_OK) {
         s->groups[hs] = grp;
       } else {
-        grp = nullptr;  // (e.g. a pool's candidate is not a persistent TMA form): each pool alone
+        grp = nullptr;  // (e.g. the first pool's candidate is not a persistent form): each pool alone
       }
     }
     if (!grp) {
