@@ -161,7 +161,8 @@ struct mcv_handle {
   // stage kernel chosen by the autotuner
   const StageLauncher *cands = nullptr;
   int ncands = 0, choice = -1;
-  bool tuned = false;  // the choice is the autotuner's, not mcv_select_tile's
+  bool tuned = false;    // the choice is the autotuner's, not mcv_select_tile's
+  bool grouped = false;  // has stepped in a group
   std::vector<float> tune_ms;
   cudaGraphExec_t graph_exec[2]{};
 };
@@ -909,9 +910,9 @@ int build_graphs(mcv_handle *h) {
   return MCV_OK;
 }
 
-// Checks the handle and lazily builds the step graphs.  With no active member
-// a step enqueues nothing (*idle); callers that need a launch pass no flag.
-int ready_to_step(mcv_handle *h, bool *idle = nullptr) {
+// Checks that the handle can step.  With no active member a step enqueues nothing
+// (*idle); callers that need a launch pass no flag.
+int check_ready(mcv_handle *h, bool *idle) {
   if (!h) return fail(MCV_ERR_ARG, "handle is NULL");
   if (!h->geometry_set) return fail(MCV_ERR_ORDER, "mcv_set_geometry must precede stepping");
   for (int k = 0; k < h->n_active; ++k)
@@ -923,7 +924,13 @@ int ready_to_step(mcv_handle *h, bool *idle = nullptr) {
     return MCV_OK;
   }
   if (idle) *idle = false;
-  return build_graphs(h);
+  return MCV_OK;
+}
+
+// ... and lazily builds the step graphs.
+int ready_to_step(mcv_handle *h, bool *idle = nullptr) {
+  if (int rc = check_ready(h, idle)) return rc;
+  return idle && *idle ? MCV_OK : build_graphs(h);
 }
 
 // After nsteps of the active members: their step counts, and (split
@@ -1932,7 +1939,7 @@ extern "C" int mcv_select_tile(mcv_handle *h, int index) {
       h->graph_exec[c] = nullptr;
     }
   h->choice = index;  // -1: autotune again before the next step
-  h->tuned = false;
+  h->tuned = h->grouped = false;
   if (index >= 0 && (int)h->tune_ms.size() != h->ncands) h->tune_ms.assign(h->ncands, -1.f);
   return MCV_OK;
 }
@@ -2020,13 +2027,17 @@ int build_group_graphs(mcv_group *g, const std::vector<mcv_handle *> &act) {
 // The handles a group step advances (those with active members) and the step
 // graph to replay first (0, or 1 when the parities are one step on), rebuilt
 // unless the handles, active counts, identity of the active lists and buffer
-// parities are the ones the graphs were built for.
+// parities are the ones the graphs were built for.  The handles' own trials and
+// graphs are left to their own first step: the group runs neither.
 int prepare_group(mcv_group *g, std::vector<mcv_handle *> &act, int &flip) {
   act.clear();
   for (mcv_handle *h : g->hs) {
     bool idle = false;
-    if (int rc = ready_to_step(h, &idle)) return rc;
-    if (!idle) act.push_back(h);
+    if (int rc = check_ready(h, &idle)) return rc;
+    if (!idle) {
+      h->grouped = true;
+      act.push_back(h);
+    }
   }
   flip = 0;
   if (act.empty()) return MCV_OK;
@@ -2082,6 +2093,9 @@ extern "C" int mcv_group_create(mcv_handle *const *handles, int count, int tile,
         h->scheme != handles[0]->scheme || h->device != handles[0]->device)
       return fail(MCV_ERR_ARG, "the handles of a group share order, precision, scheme and device");
   }
+  // a handle that has stepped in groups only has yet to choose
+  if (tile < 0 && handles[0]->choice < 0 && handles[0]->grouped)
+    if (int rc = ready_to_step(handles[0])) return rc;
   const int cand = tile >= 0 ? tile : group_form(handles[0]);
   if (cand < 0 || cand >= handles[0]->ncands || !handles[0]->cands[cand].tma)
     return fail(MCV_ERR_ARG, "the group's stage-kernel candidate must be a persistent form: TMA tiles or strips (mcv_tuning)");

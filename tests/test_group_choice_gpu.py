@@ -58,3 +58,22 @@ def test_a_handle_without_a_record_is_refused():
         api.Group(made)
     for s in made:
         s.close()
+
+
+def test_a_group_steps_handles_that_were_never_tuned():
+    """Their own trials come with their own first step; a later group that names
+    no form asks its first handle for them."""
+    made = [stepper(4, nc, "RK4", nc) for nc in (48, 20)]
+    forms = stepper(4, 48, "RK4", 48)[0].tuning()[0]
+    form = min(i for i, (shape, _) in enumerate(forms) if shape[5])
+    with api.Group([s for s, _ in made], form) as g:
+        g.step(2)
+    together = [s.get_state(0) for s, _ in made]
+    with api.Group([s for s, _ in made]) as g:
+        g.step(1)
+    for (s, st), out in zip(made, together):
+        s.select_tile(form)
+        s.set_member(0, st.phi_s, st.u, st.v, st.phi)
+        s.step(2)
+        assert same(out, s.get_state(0)), s.nc
+        s.close()
