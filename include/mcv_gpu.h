@@ -234,14 +234,15 @@ int mcv_cell_areas(int nc, double radius, double *areaCell);
 int mcv_time_steps(mcv_handle *h, int nsteps, double *ms);
 int mcv_profile_step(mcv_handle *h, int nsteps, double *stage_ms, double *halo_ms);
 
-/* Stage-kernel tile shapes the autotuner timed on this handle's grid (it runs
- * once, before the first step): ncand (at most 16) candidates,
+/* Stage-kernel tile shapes, of which the autotuner times those that can win on
+ * this handle's grid (it runs once, before the first step): ncand (at most 16) candidates,
  * shapes[6*i..] = {cells in x, cells in y, threads, sweep style (0 per-cell
  * items, n walks of n cells), CTAs per SM the kernel's registers allow, form
  * (0 one CTA per tile, 1 persistent CTAs with TMA-staged tiles or strips)}; the
  * last is the strip form, {29, 1, threads, 0, 1, 1}: one warp per strip of at most
- * 29 cells' width.  ms[i] = device time per stage with its halo kernel, *chosen =
- * the index in use.  No counterpart in the
+ * 29 cells' width.  ms[i] = device time per stage with its halo kernel, -1 if not
+ * timed (a shape that cannot win, or the only one that can), *chosen = the index in
+ * use.  No counterpart in the
  * reference (which has no GPU path). */
 int mcv_tuning(mcv_handle *h, int *ncand, int *chosen, int *shapes, float *ms);
 

@@ -402,7 +402,7 @@ class Stepper:
 
     def tuning(self):
         """Autotuner record: list of ((cells_x, cells_y, threads, walk, ctas_per_sm, persistent), ms per
-        stage with its halo kernel) and the chosen index; the last is the strip form."""
+        stage with its halo kernel, -1 if not timed) and the chosen index; the last is the strip form."""
         n, ch = ctypes.c_int(), ctypes.c_int()
         shapes = (ctypes.c_int * 96)()
         ms = (ctypes.c_float * 16)()

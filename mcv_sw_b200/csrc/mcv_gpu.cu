@@ -803,17 +803,34 @@ int enqueue_trial(mcv_handle *h, int cand, int stages) {
   return MCV_OK;
 }
 
-// Small grids: the candidates' first stages in one graph, with event records
-// between them.  Plain launches would time the host, at about 9 us a stage for
-// every form: MCV3 Nc=32 FP64 took one of 30.8 us a step where another takes 28.8.
-int time_in_graph(mcv_handle *h, const std::vector<cudaEvent_t> &ev) {
+// The forms to try on a handle's grid and active members.  The tables' upper lines
+// were drawn at large grids for the tiles that share a strip's work there; members
+// of a grid below 48 cells fill strips (29 cells) worse, and below 16 also the
+// tiles, so that all forms are tried.
+std::vector<int> forms_to_try(const mcv_handle *h) {
+  const long long cells = (long long)h->g.Nc * h->g.Nc * h->n_active;
+  std::vector<int> out;
+  if (h->g.Nc >= 16 || cells <= 3072)
+    for (int i = 0; i < h->ncands; ++i) {
+      const StageLauncher &L = h->cands[i];
+      if (cells >= L.from && (cells <= L.to || (h->g.Nc < 48 && L.to > 3072))) out.push_back(i);
+    }
+  if (out.empty())
+    for (int i = 0; i < h->ncands; ++i) out.push_back(i);
+  return out;
+}
+
+// Small grids: the forms' first two stages in one graph, with event records between
+// them.  Plain launches would time the host, at about 9 us a stage for every form:
+// MCV3 Nc=32 FP64 took one of 30.8 us a step where another takes 28.8.
+int time_in_graph(mcv_handle *h, const std::vector<int> &forms, const std::vector<cudaEvent_t> &ev) {
   MCV_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin trial capture");
   int rc = MCV_OK;
   cudaError_t e = cudaSuccess;
-  for (int i = 0; i < h->ncands && !rc && e == cudaSuccess; ++i) {
-    rc = enqueue_trial(h, i, 1);  // warm-up
+  for (size_t i = 0; i < forms.size() && !rc && e == cudaSuccess; ++i) {
+    rc = enqueue_trial(h, forms[i], 2);  // warm-up
     e = cudaEventRecordWithFlags(ev[2 * i], h->stream, cudaEventRecordExternal);
-    for (int r = 0; r < 3 && !rc; ++r) rc = enqueue_trial(h, i, 1);
+    for (int r = 0; r < 2 && !rc; ++r) rc = enqueue_trial(h, forms[i], 2);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(ev[2 * i + 1], h->stream, cudaEventRecordExternal);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -830,59 +847,68 @@ int time_in_graph(mcv_handle *h, const std::vector<cudaEvent_t> &ev) {
   }
   if (rc) return rc;
   MCV_CUDA(e, "time stage kernels");
-  for (int i = 0; i < h->ncands; ++i) {
+  for (size_t i = 0; i < forms.size(); ++i) {
     float ms = 0.f;
     MCV_CUDA(cudaEventElapsedTime(&ms, ev[2 * i], ev[2 * i + 1]), "time stage kernels");
-    h->tune_ms[i] = ms / 3.f;  // per stage
+    h->tune_ms[forms[i]] = ms / 4.f;  // per stage
   }
   return MCV_OK;
 }
 
-// Larger grids: one candidate after another, the strip form (the likely winner)
-// first; a form whose warm-up trial already takes a quarter longer than the best
-// is not timed further (MCV4 Nc=256 FP64, first step: 13.8 ms with all of them in full, 4.5 so).
-int time_in_turn(mcv_handle *h, const std::vector<cudaEvent_t> &ev) {
+// Larger grids: one form after another, the strips first; a form that takes a quarter
+// longer than the best in its first timed pass, which a pass of warm-up precedes on
+// the stream, is not timed further.
+int time_in_turn(mcv_handle *h, const std::vector<int> &forms, const std::vector<cudaEvent_t> &ev) {
   float best = 1e30f;
-  for (int i = h->ncands - 1; i >= 0; --i) {
+  for (auto i = forms.rbegin(); i != forms.rend(); ++i) {
     float ms = 0.f;
+    if (int rc = enqueue_trial(h, *i, 2)) return rc;
     for (int reps = 1; reps <= 2; ++reps) {
       cudaEventRecord(ev[0], h->stream);
       for (int r = 0; r < reps; ++r)
-        if (int rc = enqueue_trial(h, i, 2)) return rc;
+        if (int rc = enqueue_trial(h, *i, 2)) return rc;
       cudaEventRecord(ev[1], h->stream);
       MCV_CUDA(cudaEventSynchronize(ev[1]), "time stage kernels");
       MCV_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]), "time stage kernels");
       MCV_CUDA(cudaGetLastError(), "time stage kernels");
-      h->tune_ms[i] = ms / (2 * reps);  // per stage
-      if (h->tune_ms[i] > 1.25f * best) break;
+      h->tune_ms[*i] = ms / (2 * reps);  // per stage
+      if (h->tune_ms[*i] > 1.25f * best) break;
     }
-    best = std::min(best, h->tune_ms[i]);
+    best = std::min(best, h->tune_ms[*i]);
   }
   return MCV_OK;
 }
 
-// Time the candidate shapes on this grid with the first two stages of a step and
+// Time the forms that can win on this grid with the first two stages of a step and
 // the halo kernels after them, and keep the fastest: the forms overlap the halo
 // kernel to different extents, so the stage kernel's time alone does not order
 // them (MCV4 Nc=90, split precision: strips 18.8 us a stage alone and 25.5 in a
-// step, 8x8-cell tiles 19.4 and 21.8).
+// step, 8x8-cell tiles 19.4 and 21.8).  A form that is alone is taken untimed.
 int autotune(mcv_handle *h) {
   if (h->choice >= 0) return MCV_OK;
   h->tune_ms.assign(h->ncands, -1.f);
-  std::vector<cudaEvent_t> ev(2 * h->ncands, nullptr);
-  cudaError_t e = cudaSuccess;
-  for (cudaEvent_t &x : ev)
-    if (e == cudaSuccess) e = cudaEventCreate(&x);
-  int rc = e == cudaSuccess ? MCV_OK : cuda_fail(e, "event");
-  // The line: a first step of MCV3 Nc=96 FP64 (0.22 M points) takes 1.02 ms with the
-  // trials in one graph and 1.25 with them in turn; 4 members of it 2.0 and 1.6.
-  const long long points = 6LL * h->g.np * h->g.np * h->n_active;
-  if (!rc) rc = points <= 262144 ? time_in_graph(h, ev) : time_in_turn(h, ev);
-  for (cudaEvent_t x : ev)
-    if (x) cudaEventDestroy(x);
-  if (!rc) rc = check_late(h);  // a form that gave up was timed for work it did not do
-  if (rc) return rc;
-  h->choice = (int)(std::min_element(h->tune_ms.begin(), h->tune_ms.end()) - h->tune_ms.begin());
+  const std::vector<int> forms = forms_to_try(h);
+  int best = forms[0];
+  if (forms.size() > 1) {
+    std::vector<cudaEvent_t> ev(2 * forms.size(), nullptr);
+    cudaError_t e = cudaSuccess;
+    for (cudaEvent_t &x : ev)
+      if (e == cudaSuccess) e = cudaEventCreate(&x);
+    int rc = e == cudaSuccess ? MCV_OK : cuda_fail(e, "event");
+    // The line: below it launches in turn time the host and pick wrongly (MCV3 Nc=64
+    // split precision, 0.1 M points: 46.1 us a step instead of 42.7 in two of five first
+    // steps), though they take 0.06 ms less; above it both pick alike, and several
+    // members take longer in a graph (4 of MCV3 Nc=96 FP64: first step 1.04 ms, in turn 0.83).
+    const long long points = 6LL * h->g.np * h->g.np * h->n_active;
+    if (!rc) rc = points <= 262144 ? time_in_graph(h, forms, ev) : time_in_turn(h, forms, ev);
+    for (cudaEvent_t x : ev)
+      if (x) cudaEventDestroy(x);
+    if (!rc) rc = check_late(h);  // a form that gave up was timed for work it did not do
+    if (rc) return rc;
+    for (int i : forms)
+      if (h->tune_ms[i] < h->tune_ms[best]) best = i;
+  }
+  h->choice = best;
   h->tuned = true;
   return MCV_OK;
 }

@@ -18,6 +18,7 @@
 // Device layout of a padded field: [member][panel][row j][pitch P] with
 // padded indices (reference index - ips), P >= npx rounded up to 16 elements.
 #pragma once
+#include <climits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -1587,6 +1588,16 @@ struct StageLauncher {
   cudaError_t (*prepare)();      // raises the dynamic shared-memory limit of every kind
   int (*blocks_per_sm)();        // resident CTAs per SM (sizes the persistent grid)
   int strip[7];                  // strip form (mcv_strip.cuh): warps per block of each kind; else 0
+  // Cells of a launch (Nc^2 times the members) between which the autotuner tries the
+  // form: where it was within a few percent of the best, and somewhat beyond.
+  int from = 0, to = INT_MAX;
+  StageLauncher tried(int a, int b = INT_MAX) const {
+    StageLauncher l = *this;
+    l.from = a;
+    l.to = b;
+    return l;
+  }
+  StageLauncher never_tried() const { return tried(INT_MAX, 0); }
 };
 
 template <int D, int CX, int CY, int NT, int MINB, bool MIXED, int WALK, bool TMA = false, int OPT = 0>

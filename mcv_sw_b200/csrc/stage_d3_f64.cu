@@ -3,9 +3,11 @@
 // sweep style (0: per-cell items, n: walks of n cells), TMA-staged persistent
 // form) the autotuner chooses from.
 // which of them wins where (RK4 step, us; the 12x12 and 8x8 per-cell items these
-// replaced in brackets): 4x4 and 6x4 up to Nc=32 (28.8 at 32 [30.9]), 8x8 walked by
-// 448 threads at 48..64 (34.9 at 48 [38.9]), by 224 from there to 128 (62.8 at 96
-// [67.8]), strips beyond.  The TMA tiles are for groups, which run persistent forms.
+// replaced in brackets): 4x4 up to Nc=38 (28.8 at 32 [30.9], 6x4 30.8), 6x4 to 48,
+// 8x8 walked by 448 threads at 40..64 (45.8 at 64 [47.1]), by 224 from 45 to 128 (62.6
+// at 96 [67.8]; strips 68.2), 12x12 at 80 (53.5, 8x8 55.0), strips beyond (88.3 at 128,
+// 8x8 89.0).  tried(): the cells of a launch between which the autotuner times them.
+// The TMA tiles are for groups, which run persistent forms.
 #include "mcv_stage.cuh"
 
 namespace mcv {
@@ -14,13 +16,13 @@ StageLauncher strip_launcher_d3_f64();  // stage_strip_d3_f64.cu
 
 const StageLauncher *stage_launchers_d3_f64(int *count) {
   static const StageLauncher table[] = {
-    StageConfig<3, 12, 12, 320, 2, false, 2>::make(),
-    StageConfig<3, 8, 8, 224, 4, false, 2>::make(),
-    StageConfig<3, 8, 8, 448, 2, false, 2>::make(),
-    StageConfig<3, 4, 4, 224, 3, false, 0>::make(),
-    StageConfig<3, 6, 4, 224, 3, false, 0>::make(),
-    StageConfig<3, 8, 8, 224, 2, false, 0, true>::make(),
-    strip_launcher_d3_f64()};
+    StageConfig<3, 12, 12, 320, 2, false, 2>::make().tried(6000, 7500),
+    StageConfig<3, 8, 8, 224, 4, false, 2>::make().tried(2000, 65536),
+    StageConfig<3, 8, 8, 448, 2, false, 2>::make().tried(1500, 5000),
+    StageConfig<3, 4, 4, 224, 3, false, 0>::make().tried(0, 1500),
+    StageConfig<3, 6, 4, 224, 3, false, 0>::make().tried(1400, 3072),
+    StageConfig<3, 8, 8, 224, 2, false, 0, true>::make().never_tried(),
+    strip_launcher_d3_f64().tried(9000)};
   *count = (int)(sizeof(table) / sizeof(table[0]));
   return table;
 }
