@@ -20,8 +20,8 @@ def raise_flag(s):
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("device", [False, True])
 def test_late_copies_until_the_geometry_is_set_again(precision, device):
-    geom = api.Geometry(3, 8, cases.EARTH_RADIUS)
-    st, _ = cases.small(seed=2, nc=8, geom=geom)
+    geom = api.Geometry(3, 40, cases.EARTH_RADIUS)  # a grid on which several forms are timed
+    st, _ = cases.small(seed=2, nc=40, geom=geom)
 
     def start(s):
         if device:
@@ -30,7 +30,7 @@ def test_late_copies_until_the_geometry_is_set_again(precision, device):
             s.set_geometry(geom)
         s.set_member(0, st.phi_s, st.u, st.v, st.phi)
 
-    with api.Stepper(3, 8, st.dt, "RK4", precision=precision, radius=cases.EARTH_RADIUS) as s:
+    with api.Stepper(3, 40, st.dt, "RK4", precision=precision, radius=cases.EARTH_RADIUS) as s:
         start(s)
         s.step(2)
         raise_flag(s)
