@@ -16,7 +16,7 @@ SOURCES = ["mcv_gpu.cu", "stage_d3_f64.cu", "stage_d3_mix.cu", "stage_d4_f64.cu"
 # per-source flags: the device geometry restates host formulas compiled
 # without FMA contraction; the strip kernels write their fused operations out
 SOURCE_FLAGS = {src: ["-fmad=false"] for src in SOURCES if src == "mcv_geometry.cu" or src.startswith("stage_strip_")}
-HEADERS = ["mcv_stage.cuh", "mcv_strip.cuh", "mcv_strip64.cuh", "mcv_strip_table.cuh", "mcv_halo.cuh", "mcv_tma.cuh", "mcv_ksum.cuh", "mcv_internal.h", os.path.join("..", "..", "include", "mcv_gpu.h")]
+HEADERS = ["mcv_stage.cuh", "mcv_cut.h", "mcv_strip.cuh", "mcv_strip64.cuh", "mcv_strip_table.cuh", "mcv_halo.cuh", "mcv_tma.cuh", "mcv_ksum.cuh", "mcv_internal.h", os.path.join("..", "..", "include", "mcv_gpu.h")]
 OBJ_DIR = os.path.join(HERE, "_lib", "obj")
 
 NVCC_FLAGS = [

@@ -660,100 +660,6 @@ void number_items(StageBatch<NB> &b, int n) {
   b.total = nin + ned;
 }
 
-// Divides the columns of a strip-form launch over b's first n grids between
-// `warps` resident warps (StageBatch, mcv_strip.cuh).  The cost of a cut is that of
-// its longest warp, in cell rows, a strip paying kStart for its start and halo rows.
-//  - Segments of about the same number of cell rows in every column, as many as
-//    cost least.
-//  - Segments of two lengths, where that costs 5% less and there are several
-//    members: whole passes of long segments for some of the panels, then short ones
-//    for the others.  64 members of MCV3 Nc=128 take whole columns for 355 panels
-//    and twelfths for 29 instead of 16ths for all: RK4 2.37 -> 2.19 ms/step split
-//    precision; 50 of Nc=100 FP64 1.51 -> 1.32.  Where less is promised or panels
-//    are few and large it was lost (MCV4 Nc=700 FP64: 2.98 -> 3.16).
-//  - One run per warp, where that costs 4% less and neighbouring columns stay in
-//    step: they share sectors at their seams, which are read twice where the
-//    neighbour's are no longer in L2.  What a stage touches (76 bytes a point, FP64
-//    130) stays there up to 126 MB (4 members of MCV3 Nc=128 split precision: RK4
-//    180 -> 169 us).  Other grids want a column to be a whole number of runs (MCV4
-//    Nc=256 FP64, 10.96: RK3 283 -> 276 us; Nc=280, 9.87: RK4 551 -> 596; 4 members
-//    of MCV3 Nc=181 split precision, 10.57: 275 -> 306) and runs to be short (MCV3
-//    Nc=512 FP64, 47 rows, 10.96: 738 -> 827).
-template <int NB>
-int cut_strips(StageBatch<NB> &b, int n, int warps) {
-  constexpr double kStart = (double)kStripStart / kStripUnit;
-  constexpr long long kLongRun = 32;  // cell rows
-  long long units = 0, rows = 0, points = 0;
-  int most = 1;
-  for (int k = 0; k < n; ++k) {
-    b.nsx[k] = (b.g[k].Nc + kStripCells - 1) / kStripCells;
-    const long long columns = 6LL * b.slots[k] * b.nsx[k];
-    units += columns * (b.g[k].Nc * kStripUnit + kStripStart);
-    rows += columns * b.g[k].Nc;
-    points += 6LL * b.slots[k] * b.g[k].n * b.g[k].n;
-    most = std::max(most, b.g[k].Nc);
-  }
-  if (units > INT_MAX / 2) return fail(MCV_ERR_ARG, "too many cell rows for one launch");
-  double best = 1e300;
-  int len = 1;
-  for (int l = 1; l <= most; ++l) {
-    long long strips = 0;
-    for (int k = 0; k < n; ++k) strips += 6LL * b.slots[k] * b.nsx[k] * ((b.g[k].Nc + l - 1) / l);
-    const double cost = (double)((strips + warps - 1) / warps) * (l + kStart);
-    if (cost < best) {
-      best = cost;
-      len = l;
-    }
-  }
-  int pm1 = 0, sy1 = 0, sy2 = 0;
-  if (n == 1 && b.slots[0] > 1) {
-    const int Nc = b.g[0].Nc, nsx = b.nsx[0], per = 6 * b.slots[0];
-    double split = 0.95 * best;
-    for (int s1 = 1; s1 <= Nc; ++s1) {
-      const long long strip = (long long)nsx * s1;  // strips of a panel
-      const int passes = (int)(per * strip / warps), m = (int)((long long)passes * warps / strip);
-      if (m <= 0 || m >= per) continue;
-      const double long1 = passes * ((Nc + s1 - 1) / s1 + kStart);
-      if (long1 >= split) continue;
-      for (int p2 = 1; p2 <= 3; ++p2) {
-        const int s2 = (int)std::min<long long>(Nc, (long long)p2 * warps / ((long long)(per - m) * nsx));
-        if (s2 < 1) continue;
-        const double cost = long1 + p2 * ((Nc + s2 - 1) / s2 + kStart);
-        if (cost < split) {
-          split = cost;
-          pm1 = m;
-          sy1 = s1;
-          sy2 = s2;
-        }
-      }
-    }
-    if (pm1) best = split;
-  }
-  const long long run = (units + (long long)warps * kStripUnit - 1) / ((long long)warps * kStripUnit);  // cell rows, up
-  bool runs = run <= kLongRun && (double)run + kStart < 0.96 * best;
-  const bool cached = points * (b.a[0].rsg ? 130 : 76) <= (126ll << 20);
-  for (int k = 0; k < n && !cached; ++k) {
-    const double per_column = (double)(b.g[k].Nc * kStripUnit + kStripStart) * warps / (double)units;
-    runs = runs && std::abs(per_column - std::round(per_column)) <= 0.1;
-  }
-  b.ngrids = n;
-  int at = 0;
-  for (int k = 0; k < n; ++k) {
-    const int columns = 6 * b.slots[k] * b.nsx[k];
-    b.t0[k] = at;
-    b.pm1[k] = pm1 ? pm1 : 6 * b.slots[k];
-    b.sy[k] = runs ? 0 : pm1 ? sy1 : (b.g[k].Nc + len - 1) / len;
-    b.sy2[k] = sy2;
-    at += runs ? columns * (b.g[k].Nc * kStripUnit + kStripStart)
-               : b.pm1[k] * b.nsx[k] * b.sy[k] + (6 * b.slots[k] - b.pm1[k]) * b.nsx[k] * sy2;
-  }
-  b.t0[n] = at;
-  b.total = runs ? (int)std::min<long long>(warps, rows) : at;
-  b.run_q = at / b.total;
-  b.run_r = at % b.total;
-  return MCV_OK;
-}
-
 // Blocks of a persistent launch over b's first n grids, whose work it numbers (0: error).
 template <int NB>
 int plan_persistent(StageBatch<NB> &b, int n, const StageLauncher &L, int kind, int resident) {
@@ -762,7 +668,10 @@ int plan_persistent(StageBatch<NB> &b, int n, const StageLauncher &L, int kind, 
     number_items(b, n);
     return std::max(1, std::min(b.total, resident));
   }
-  if (cut_strips(b, n, resident * wpb)) return 0;
+  if (!cut_strips(b, n, resident * wpb, b.a[0].rsg ? 130 : 76)) {
+    fail(MCV_ERR_ARG, "too many cell rows for one launch");
+    return 0;
+  }
   return std::max(1, std::min(b.total, resident));
 }
 

@@ -24,6 +24,7 @@
 
 #include <type_traits>
 
+#include "mcv_cut.h"
 #include "mcv_tma.cuh"
 
 namespace mcv {
@@ -94,13 +95,9 @@ struct StageArgs {
 // that with programmatic dependent launch the edge-free items of every grid
 // start while the previous halo kernels still run.
 constexpr int kMaxGrids = 4;
-// strip form: owned cells per strip, lanes 1..29 (lane 31 lends its first point to lane 30)
-constexpr int kStripCells = 29;
-// What a strip pays for its start and its two halo rows, in cell rows: 2.25
-// (measured: MCV4 Nc=256 stages fit (rows + 2.2) x 3.6 us split precision)
-constexpr int kStripUnit = 8, kStripStart = 18;
 template <int NB>
 struct StageBatch {
+  static constexpr int kGrids = NB;
   TileMaps tm[NB];  // tensor maps of each grid's staged fields (TMA form)
   GridDesc g[NB];
   StageArgs a[NB];
@@ -110,13 +107,7 @@ struct StageBatch {
   int in0[NB + 1];  // first edge-free item of each grid
   int ed0[NB + 1];  // first edge item of each grid, counted from nin
   int slots[NB];    // active members of each grid
-  // strip form: nsx columns of at most kStripCells cells across a panel.  Either
-  // (sy > 0) the columns of the first pm1 panels (of all members) are cut into sy
-  // segments of cell rows, those of the others into sy2, total strips in all, the
-  // first of a grid t0; or `total` runs of equal length share the columns
-  // of every grid laid end to end, kStripUnit units a cell row and kStripStart in
-  // front of each column, from unit t0 of a grid on: run id starts at
-  // id run_q + id run_r / total.
+  // strip form: its cut (mcv_cut.h)
   int nsx[NB], sy[NB], sy2[NB], pm1[NB], t0[NB + 1];
   int run_q, run_r;
 };

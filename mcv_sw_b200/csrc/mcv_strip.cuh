@@ -51,63 +51,6 @@ __device__ __forceinline__ void hand_to_copies() {
   __syncwarp();
 }
 
-// A strip: cells [c0, c0 + w) of cell rows [r0, r1) of one panel of one active
-// member.  A warp takes, one after the other,
-//  - segments of columns, cut alike over many panels: neighbouring columns are
-//    worked on at the same rows at the same time, so that a row of a field is read
-//    as a whole (panels fastest: split precision's six panels share the metric
-//    planes); or
-//  - a run of the columns laid end to end: the end of a column and the beginning
-//    of another, so that no warp is left over.
-// Which, the host decides (cut_strips).
-struct Strip {
-  int c0, w, r0, r1, panel, slot;
-};
-template <int NB>
-__device__ __forceinline__ void strip_column(const StageBatch<NB> &b, int k, int pm, int col, Strip &t) {
-  const int Nc = b.g[k].Nc, nsx = b.nsx[k];
-  t.slot = pm / 6;
-  t.panel = pm - 6 * t.slot;
-  t.c0 = Nc * col / nsx;
-  t.w = Nc * (col + 1) / nsx - t.c0;
-}
-// The next strip of the warp whose work is item id, [x, xe) of it left (grid k);
-// x moves past it.  False if the run holds no cell row of that column.
-template <int NB>
-__device__ __forceinline__ bool next_strip(const StageBatch<NB> &b, int id, int &x, int xe, int &k, Strip &t) {
-  const bool segments = b.sy[0] > 0;
-  const int at = segments ? id : x;
-  k = 0;
-#pragma unroll
-  for (int j = 1; j < NB; ++j)
-    if (j < b.ngrids && at >= b.t0[j]) k = j;
-  const int Nc = b.g[k].Nc, nsx = b.nsx[k];
-  if (segments) {
-    int local = id - b.t0[k], pm = 0, per = b.pm1[k], sy = b.sy[k];
-    const int first = per * nsx * sy;
-    if (local >= first) {
-      local -= first;
-      pm = per;
-      per = 6 * b.slots[k] - per;
-      sy = b.sy2[k];
-    }
-    const int q = local / per, seg = q / nsx;
-    strip_column(b, k, pm + local - q * per, q - seg * nsx, t);
-    t.r0 = Nc * seg / sy;
-    t.r1 = Nc * (seg + 1) / sy;
-    x = xe;
-    return true;
-  }
-  const int len = Nc * kStripUnit + kStripStart;
-  const int column = (x - b.t0[k]) / len, start = b.t0[k] + column * len, pm = column / nsx;
-  strip_column(b, k, pm, column - pm * nsx, t);
-  auto row = [&](int y) { return max(0, y - start - kStripStart + kStripUnit / 2) / kStripUnit; };
-  t.r0 = row(x);
-  x = min(xe, start + len);
-  t.r1 = row(x);
-  return t.r1 > t.r0;
-}
-
 // Shared memory of one warp for stage kind KIND: the staged input of a cell row
 // ([field][H rows][RE] each), the operands and results of the update of the
 // cell row before, the strip's metric entries in x, and the x sweep's results.
@@ -287,9 +230,8 @@ __global__ void __launch_bounds__(32 * StripSmem<D, KIND>::WPB, 1) strip_kernel(
 
   // runs are dealt to the blocks in turn, so that few of them use every SM
   for (int id = warp * gridDim.x + blockIdx.x; id < b.total; id += stride) {
-  // (segments: run_q = 1, run_r = 0)
-  int x = id * b.run_q + (int)((long long)id * b.run_r / b.total);
-  const int xe = (id + 1) * b.run_q + (int)((long long)(id + 1) * b.run_r / b.total);
+  int x, xe;
+  strip_work(b, id, x, xe);
   while (x < xe) {
     int k;
     Strip st;

@@ -101,9 +101,8 @@ __global__ void __launch_bounds__(32 * Strip64Smem<D, KIND>::WPB, 1)
 
   // runs are dealt to the blocks in turn, so that few of them use every SM
   for (int id = warp * gridDim.x + blockIdx.x; id < b.total; id += stride) {
-  // (segments: run_q = 1, run_r = 0)
-  int x = id * b.run_q + (int)((long long)id * b.run_r / b.total);
-  const int xe = (id + 1) * b.run_q + (int)((long long)(id + 1) * b.run_r / b.total);
+  int x, xe;
+  strip_work(b, id, x, xe);
   while (x < xe) {
     int k;
     Strip st;
