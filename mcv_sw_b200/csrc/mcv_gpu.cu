@@ -684,12 +684,12 @@ int launch_stage(mcv_handle *h, int cand, int s, int c) {
   const StageLaunchFn launch = h->active_ident ? L.launch_ident[kind] : L.launch[kind];
   if (!L.tma) {
     number_items(b, 1);
-    launch(dim3(b.g[0].tiles_x * b.g[0].tiles_y, 6, h->n_active), h->stream, b, true);
+    launch(dim3(b.g[0].tiles_x * b.g[0].tiles_y, 6, h->n_active), h->stream, b);
     return MCV_OK;
   }
   const int ctas = plan_persistent(b, 1, L, kind, h->bps[cand] * h->nsm);
   if (!ctas) return MCV_ERR_ARG;
-  launch(dim3(ctas), h->stream, b, true);
+  launch(dim3(ctas), h->stream, b);
   return MCV_OK;
 }
 
@@ -1920,7 +1920,7 @@ int enqueue_group_stage(mcv_group *g, const std::vector<mcv_handle *> &act, cons
     if (int rc = add_grid(b, (int)k, act[k], L, s, curs[k])) return rc;
   const int ctas = plan_persistent(b, (int)act.size(), L, stage_kind(act[0], s), g->bps * act[0]->nsm);
   if (!ctas) return MCV_ERR_ARG;
-  L.launch_batch[stage_kind(act[0], s)](dim3(ctas), g->stream, b, true);
+  L.launch_batch[stage_kind(act[0], s)](dim3(ctas), g->stream, b);
   launch_halo_batch<kMaxGrids>(act.data(), curs.data(), (int)act.size(), s, g->stream);
   return MCV_OK;
 }

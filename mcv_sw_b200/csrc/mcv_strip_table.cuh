@@ -16,7 +16,7 @@ struct StripConfig {
     else return &strip64_kernel<D, KIND, NB, IDENT>;
   }
   template <int KIND, int NB, bool IDENT>
-  static void launch_nb(dim3 grid, cudaStream_t s, const StageBatch<NB> &b, bool pdl) {
+  static void launch_nb(dim3 grid, cudaStream_t s, const StageBatch<NB> &b) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(32 * S<KIND>::WPB);
@@ -26,20 +26,20 @@ struct StripConfig {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel<KIND, NB, IDENT>(), b);
   }
   template <int KIND>
-  static void launch(dim3 grid, cudaStream_t s, const StageBatch<1> &b, bool pdl) {
-    launch_nb<KIND, 1, false>(grid, s, b, pdl);
+  static void launch(dim3 grid, cudaStream_t s, const StageBatch<1> &b) {
+    launch_nb<KIND, 1, false>(grid, s, b);
   }
   template <int KIND>
-  static void launch_ident(dim3 grid, cudaStream_t s, const StageBatch<1> &b, bool pdl) {
-    launch_nb<KIND, 1, true>(grid, s, b, pdl);
+  static void launch_ident(dim3 grid, cudaStream_t s, const StageBatch<1> &b) {
+    launch_nb<KIND, 1, true>(grid, s, b);
   }
   template <int KIND>
-  static void launch_batch(dim3 grid, cudaStream_t s, const StageBatch<kMaxGrids> &b, bool pdl) {
-    launch_nb<KIND, kMaxGrids, false>(grid, s, b, pdl);
+  static void launch_batch(dim3 grid, cudaStream_t s, const StageBatch<kMaxGrids> &b) {
+    launch_nb<KIND, kMaxGrids, false>(grid, s, b);
   }
   template <int KIND>
   static cudaError_t attr() {
