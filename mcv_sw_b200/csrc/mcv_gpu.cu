@@ -2013,6 +2013,16 @@ int group_form(const mcv_handle *h) {
   return best;
 }
 
+// ... of a handle that has stepped in groups only and cannot run its trials now (no
+// active member, or one not set): the last persistent form tried on its grid with all
+// members, -1 where none is.
+int untimed_form(const mcv_handle *h) {
+  const long long cells = (long long)h->g.Nc * h->g.Nc * h->members;
+  for (int i = h->ncands - 1; i >= 0; --i)
+    if (h->cands[i].tma && cells >= h->cands[i].from && cells <= h->cands[i].to) return i;
+  return -1;
+}
+
 }  // namespace
 
 extern "C" int mcv_group_create(mcv_handle *const *handles, int count, int tile, mcv_group **out) {
@@ -2028,10 +2038,16 @@ extern "C" int mcv_group_create(mcv_handle *const *handles, int count, int tile,
         h->scheme != handles[0]->scheme || h->device != handles[0]->device)
       return fail(MCV_ERR_ARG, "the handles of a group share order, precision, scheme and device");
   }
-  // a handle that has stepped in groups only has yet to choose
-  if (tile < 0 && handles[0]->choice < 0 && handles[0]->grouped)
-    if (int rc = ready_to_step(handles[0])) return rc;
-  const int cand = tile >= 0 ? tile : group_form(handles[0]);
+  int cand = tile;
+  if (tile < 0) {
+    // a handle that has stepped in groups only has yet to choose
+    mcv_handle *h = handles[0];
+    bool idle = false;
+    const bool choose = h->choice < 0 && h->grouped, able = choose && check_ready(h, &idle) == MCV_OK && !idle;
+    if (able)
+      if (int rc = autotune(h)) return rc;
+    cand = choose && !able ? untimed_form(h) : group_form(h);
+  }
   if (cand < 0 || cand >= handles[0]->ncands || !handles[0]->cands[cand].tma)
     return fail(MCV_ERR_ARG, "the group's stage-kernel candidate must be a persistent form: TMA tiles or strips (mcv_tuning)");
   mcv_group *g = new mcv_group();

@@ -77,3 +77,18 @@ def test_a_group_steps_handles_that_were_never_tuned():
         s.step(2)
         assert same(out, s.get_state(0)), s.nc
         s.close()
+
+
+def test_a_group_of_handles_that_were_never_tuned_and_rest():
+    """No member of the first handle is active, so it has nothing to time."""
+    made = [stepper(4, nc, "RK4", nc) for nc in (48, 20)]
+    tile = min(i for i, (shape, _) in enumerate(stepper(4, 48, "RK4", 48)[0].tuning()[0]) if shape[5])
+    with api.Group([s for s, _ in made], tile) as g:
+        g.step(1)
+    made[0][0].set_active([])
+    rests, steps = [s.get_state(0) for s, _ in made]
+    with api.Group([s for s, _ in made]) as g:
+        g.step(2)
+    assert same(rests, made[0][0].get_state(0)) and not same(steps, made[1][0].get_state(0))
+    for s, _ in made:
+        s.close()
