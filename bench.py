@@ -184,6 +184,12 @@ def measured_peak():
         return DEFAULT_HBM_GBS, "fallback"
 
 
+def stage_kernel_name(shape, precision):
+    """The stage kernel of a candidate shape: the strip form is one cell row high."""
+    form = "stage_kernel" if shape[1] > 1 else "strip64_kernel" if precision == "fp64" else "strip_kernel"
+    return f"{form} ({precision})"
+
+
 def stage_traffic_per_pv():
     """DRAM bytes per interior PV per stage-kernel launch from the committed ncu
     summary (profiles/stage_kernel_traffic.txt: `<workload> <kind> <bytes_per_pv>`)."""
@@ -459,7 +465,7 @@ def run_ours(args):
     nst = len(head["stage_ms"])
     roofline = {"bound": "hbm", "achieved": head["achieved_gbs"], "peak": peak, "unit": "GB/s",
                 "frac": head["achieved_gbs"] / peak, "traffic": traffic, "peak_source": peak_kind,
-                "kernel": f"stage_kernel ({args.precision})",
+                "kernel": stage_kernel_name(head["tile"]["chosen"], args.precision),
                 "algorithmic_bytes_per_launch": head["bytes_per_pv_step"] * n_pv / nst,
                 "stage_ms": head["stage_ms"], "halo_ms": head["halo_ms"],
                 "halo_share_of_step": nst * head["halo_ms"] / head["ms_per_step"]}

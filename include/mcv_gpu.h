@@ -361,8 +361,8 @@ int mcv_server_stats(mcv_server *s, long long *stats);
  * batched launch (mcv_group_*), and a pool whose class has a chunk on the GPU
  * waits for it (at most one chunk) so that the class starts together.
  * max_grids = 1 (the default): every pool on its own stream.  A grouped chunk
- * takes the fewest steps any of its forecasts has left.  Pools whose
- * stage-kernel candidate is not a persistent TMA form step alone.
+ * takes the fewest steps any of its forecasts has left.  Pools whose first
+ * grid has no persistent form for the group (mcv_group_create) step alone.
  * *grouped_chunks (may be NULL): grouped chunks launched so far. */
 int mcv_server_set_grouping(mcv_server *s, int max_grids, double max_cost_ratio, long long *grouped_chunks);
 
