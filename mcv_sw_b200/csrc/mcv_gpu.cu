@@ -822,6 +822,8 @@ int autotune(mcv_handle *h) {
   return MCV_OK;
 }
 
+// One step a graph: graphs run one after the other, on which the halo kernel's early
+// reads of Y rely (mcv_halo.cuh).
 int build_graphs(mcv_handle *h) {
   if (h->graph_exec[0]) return MCV_OK;
   if (int rc = autotune(h)) return rc;

@@ -243,6 +243,8 @@ __global__ void __launch_bounds__(kHaloSeg * D) halo_kernel(const __grid_constan
   // before the stage kernel that writes the increments, boundary copies and
   // (FP64 form) the state has completed: everything above reads only what it
   // leaves alone (the strip tables, the active list and, split precision, Y).
+  // That stage kernel may itself be waiting for the halo kernel before it, which
+  // must not write Y either: only a step's last one does, and a step ends its graph.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // the next stage kernel may launch now (the stage kernel before this one
   // has completed): its items clear of the panel edges read nothing this
